@@ -352,6 +352,7 @@ void RenderBatch(MuonBatch *b, const MuonRenderParams *params, double *const *d_
   const BatchScene *d_scenes = b->scene_table.as<BatchScene>();
   const BatchSeg *d_segs = b->seg_table.as<BatchSeg>();
   uint64_t launches = 0;
+  const int tree_nodes = static_cast<int>(b->total_nodes / static_cast<uint64_t>(n));  // of one scene, on average
   auto enqueue = [&]() {
     CUDA_TRY(cudaMemsetAsync(b->counters.ptr, 0, stride * waves.size() * sizeof(uint32_t), st));
     CUDA_TRY(cudaMemsetAsync(b->stats.ptr, 0, sizeof(unsigned long long) * kNumStats, st));
@@ -362,12 +363,12 @@ void RenderBatch(MuonBatch *b, const MuonRenderParams *params, double *const *d_
       LaunchCameraBatch(d_scenes, wsegs, w.nseg, w.paths, pb, wc, st);
       ++launches;
       for (int k = 0; k < w.bounces; ++k) {
-        LaunchExtend(b->dev, pb, wc, k, w.paths, isect, stats_on, st);
+        LaunchExtend(b->dev, pb, wc, k, w.paths, isect, stats_on, tree_nodes, st);
         LaunchShadePathBatch(b->dev, d_scenes, wsegs, S, isect, pb, wc, k, w.paths, st);
         launches += 2;
         if (S > 0) {
           LaunchOcclude(b->dev, pb, wc, k, S, static_cast<int>(std::min<int64_t>(int64_t(w.paths) * S, INT32_MAX)),
-                        isect, stats_on, st);
+                        isect, stats_on, tree_nodes, st);
           ++launches;
         }
         LaunchFold(pb, wc, k, S, w.paths, st);

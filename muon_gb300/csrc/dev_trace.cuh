@@ -509,12 +509,18 @@ __device__ __forceinline__ bool TravRun(const DevScene &s, RayPre &r, TravState 
 // with postponed leaves): a lane that reaches a leaf keeps it aside and
 // descends further from its stack until every lane still descending holds a
 // leaf, so that the warp tests leaves together instead of serialising inner
-// nodes of some lanes against leaves of others. Every leaf reached is tested;
-// only the order changes (exact-distance ties may resolve differently).
+// nodes of some lanes against leaves of others. Every leaf reached is tested,
+// in each lane's own order.
+//
+// A ray of a deep tree takes dozens of nodes from leaf to leaf, and a warp that
+// waits for its slowest lane descends with 9 of 32 lanes (dense mesh, 56 nodes
+// and two leaves per ray). So the descent also ends when fewer than
+// kMinDescend lanes are left in it: the others test their leaves, or take new
+// rays, and all go on together. 0 leaves the check out.
 #ifndef MUON_SPECULATIVE
 #define MUON_SPECULATIVE 1
 #endif
-template <bool kAnyHit, bool kStats, int kTriTest>
+template <bool kAnyHit, bool kStats, int kTriTest, int kMinDescend>
 __device__ __forceinline__ bool TravRunSpeculative(const DevScene &s, RayPre &r, TravState &t, TraceCounters *cnt,
                                                    bool *overflow, int min_active) {
   if (s.num_nodes == 0) return true;
@@ -560,7 +566,8 @@ __device__ __forceinline__ bool TravRunSpeculative(const DevScene &s, RayPre &r,
         leaf = t.node;  // postpone this leaf and keep descending
         next();
       }
-      if (!__any_sync(__activemask(), leaf == 0)) break;
+      const unsigned descending = __activemask();
+      if ((kMinDescend > 0 && __popc(descending) < kMinDescend) || !__any_sync(descending, leaf == 0)) break;
     }
     // the postponed leaf, then the current node for as long as it is a leaf
     if (leaf == 0 && t.node < 0 && t.node != kEmptyLink) {

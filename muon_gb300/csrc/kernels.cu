@@ -341,12 +341,22 @@ __global__ void __launch_bounds__(kBlock) CameraBatchKernel(const BatchScene *sc
 #define MUON_REFILL_THRESHOLD 24
 #endif
 constexpr int kRefillThreshold = MUON_REFILL_THRESHOLD;
+// Lanes below which a warp leaves the descent (TravRunSpeculative), for trees of
+// at least kDeepNodes nodes. Extend + occlude ms of dense-mesh frames without and
+// with, by nodes: 512x512x16 6.70 / 6.72 (1,737), 7.32 / 7.21 (3,959), 8.02 / 7.91
+// (12,878), 12.20 / 11.43 (52,694), 13.39 / 12.44 (195,485); 1024x1024x16 84.2 /
+// 74.4 (773,807); there 8, 12 and 20 lanes give 78.1, 75.6 and 74.6. Shallow trees
+// lose, their lanes reach leaves together: sphere field (448 nodes) 1.99 / 2.17,
+// Cornell box 0.80 / 0.89; and so do batches of small trees (eight of 1,000 to
+// 10,000 triangles: 7.95 / 8.10 ms).
+constexpr int kDeepMinDescend = 16;
+constexpr int kDeepNodes = 8192;
 // Minimum resident blocks per SM the traversal kernels are compiled for.
 #ifndef MUON_TRAVERSAL_MIN_BLOCKS
 #define MUON_TRAVERSAL_MIN_BLOCKS 4
 #endif
 
-template <bool kAnyHit, bool kStats, int kMode, class Load, class Finish>
+template <bool kAnyHit, bool kStats, int kMode, bool kDeep, class Load, class Finish>
 __device__ __forceinline__ void PersistentTraverse(const DevScene &s, int n, uint32_t *fetch, Load load,
                                                    Finish finish, TraceCounters &c, bool &overflow) {
   const int lane = threadIdx.x & 31;
@@ -385,8 +395,8 @@ __device__ __forceinline__ void PersistentTraverse(const DevScene &s, int n, uin
       }
     }
     if (!__any_sync(0xffffffffu, ray >= 0)) break;
-    if (ray >= 0 && (MUON_SPECULATIVE ? TravRunSpeculative<kAnyHit, kStats, kMode>(s, r, t, &c, &overflow,
-                                                                                    kRefillThreshold)
+    if (ray >= 0 && (MUON_SPECULATIVE ? TravRunSpeculative<kAnyHit, kStats, kMode, kDeep ? kDeepMinDescend : 0>(
+                                          s, r, t, &c, &overflow, kRefillThreshold)
                                       : TravRun<kAnyHit, kStats, kMode>(s, r, t, &c, &overflow, kRefillThreshold))) {
       finish(ray, t);
       ray = -1;
@@ -409,14 +419,14 @@ __device__ __forceinline__ void PersistentTraverse(const DevScene &s, int n, uin
 #define MUON_STABLE_CLASSES 1
 #endif
 
-template <bool kStats, int kTri>
+template <bool kStats, int kTri, bool kDeep>
 __global__ void __launch_bounds__(kBlock, MUON_TRAVERSAL_MIN_BLOCKS) ExtendKernel(DevScene s, PathBuffers b, WaveCounters wc, int bounce) {
   const int n = static_cast<int>(*wc.count(bounce));
   const float4 *__restrict__ ray_o = Pick(b.ray_o, bounce & 1);
   const float4 *__restrict__ ray_d = Pick(b.ray_d, bounce & 1);
   TraceCounters c;
   bool overflow = false;
-  PersistentTraverse<false, kStats, kTri>(
+  PersistentTraverse<false, kStats, kTri, kDeep>(
       s, n, wc.fetch_extend(bounce),
       [&](int j, float3 *o, float3 *d, float *tmax, int *root) {
         float4 o4 = ray_o[j], d4 = ray_d[j];
@@ -568,13 +578,13 @@ __global__ void __launch_bounds__(kClassThreads) ClassScatterKernel(PathBuffers 
 
 // Shadow queue entries are slot indices (entry * S + slot). A blocked slot's
 // contribution is zeroed.
-template <bool kStats, int kTri>
+template <bool kStats, int kTri, bool kDeep>
 __global__ void __launch_bounds__(kBlock, MUON_TRAVERSAL_MIN_BLOCKS) OccludeKernel(DevScene s, PathBuffers b, WaveCounters wc, int bounce,
                                                         int slots) {
   const int n = static_cast<int>(*wc.shadow(bounce));
   TraceCounters c;
   bool overflow = false;
-  PersistentTraverse<true, kStats, kTri>(
+  PersistentTraverse<true, kStats, kTri, kDeep>(
       s, n, wc.fetch_occlude(bounce),
       [&](int j, float3 *o, float3 *d, float *tmax, int *root) {
         uint32_t slot = b.shq[j];
@@ -1535,7 +1545,7 @@ void SetTraversalGrid(int sms) {
   // Enough resident blocks to fill every SM once; the persistent traversal
   // kernels hand out rays themselves.
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ExtendKernel<false, MUON_ISECT_EXACT>, kBlock, 0) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ExtendKernel<false, MUON_ISECT_EXACT, true>, kBlock, 0) !=
           cudaSuccess ||
       per_sm < 1)
     per_sm = 4;
@@ -1558,13 +1568,14 @@ void LaunchCamera(const DevCamera &cam, const WaveInfo &w, const PathBuffers &b,
 }
 
 void LaunchExtend(const DevScene &s, const PathBuffers &b, WaveCounters wc, int bounce, int bound, int isect,
-                  bool stats, cudaStream_t st) {
+                  bool stats, int tree_nodes, cudaStream_t st) {
   if (bound <= 0) return;
   WithMode(isect, [&](auto m) {
     constexpr int M = decltype(m)::value;
     const unsigned g = TraversalBlocks(bound);
-    if (stats) ExtendKernel<true, M><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
-    else ExtendKernel<false, M><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
+    if (stats) ExtendKernel<true, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
+    else if (tree_nodes >= kDeepNodes) ExtendKernel<false, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
+    else ExtendKernel<false, M, false><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
   });
   if (MUON_STABLE_CLASSES) {
     const unsigned tiles = static_cast<unsigned>((bound + kClassTile - 1) / kClassTile);
@@ -1602,13 +1613,14 @@ void LaunchShadePath(const DevScene &s, const WaveInfo &w, const ShadeParams &sp
 }
 
 void LaunchOcclude(const DevScene &s, const PathBuffers &b, WaveCounters wc, int bounce, int slots, int bound,
-                   int isect, bool stats, cudaStream_t st) {
+                   int isect, bool stats, int tree_nodes, cudaStream_t st) {
   if (bound <= 0 || slots <= 0) return;
   WithMode(isect, [&](auto m) {
     constexpr int M = decltype(m)::value;
     const unsigned g = TraversalBlocks(bound);
-    if (stats) OccludeKernel<true, M><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
-    else OccludeKernel<false, M><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
+    if (stats) OccludeKernel<true, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
+    else if (tree_nodes >= kDeepNodes) OccludeKernel<false, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
+    else OccludeKernel<false, M, false><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
   });
 }
 

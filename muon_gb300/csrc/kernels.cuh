@@ -134,8 +134,10 @@ void SetPersistentGrid(int blocks);
 void SetTraversalGrid(int sms);
 
 void LaunchCamera(const DevCamera &cam, const WaveInfo &w, const PathBuffers &b, WaveCounters wc, cudaStream_t st);
+// tree_nodes: nodes of one scene's BVH (the mean over a batch), which picks the
+// traversal kernels' variant.
 void LaunchExtend(const DevScene &s, const PathBuffers &b, WaveCounters wc, int bounce, int bound, int isect,
-                  bool stats, cudaStream_t st);
+                  bool stats, int tree_nodes, cudaStream_t st);
 void LaunchShadeDebug(const DevScene &s, const PathBuffers &b, WaveCounters wc, int integrator, int bound, int isect,
                       cudaStream_t st);
 // Raytracer / AnalyticDirect for every path of a wave; rays are traced up to
@@ -145,7 +147,7 @@ void LaunchWhitted(const DevScene &s, const PathBuffers &b, const WaveInfo &w, i
 void LaunchShadePath(const DevScene &s, const WaveInfo &w, const ShadeParams &sp, const PathBuffers &b,
                      WaveCounters wc, int bounce, int bound, cudaStream_t st);
 void LaunchOcclude(const DevScene &s, const PathBuffers &b, WaveCounters wc, int bounce, int slots, int bound,
-                   int isect, bool stats, cudaStream_t st);
+                   int isect, bool stats, int tree_nodes, cudaStream_t st);
 void LaunchFold(const PathBuffers &b, WaveCounters wc, int bounce, int slots, int bound, cudaStream_t st);
 void LaunchFilm(const WaveInfo &w, const PathBuffers &b, double *sum, double *sum_sq, uint32_t *count,
                 cudaStream_t st);

@@ -180,7 +180,7 @@ extern "C" int muon_gpu_render_noalloc(MuonScene *scene, const MuonRenderParams 
     WaveCounters wc{counters};
     LaunchCamera(*v.cam, w, b, wc, st);
     for (int k = 0; k < bp.bounces; ++k) {
-      LaunchExtend(*v.dev, b, wc, k, w.n, p.intersect_mode, stats_on, st);
+      LaunchExtend(*v.dev, b, wc, k, w.n, p.intersect_mode, stats_on, v.dev->num_nodes, st);
       if (!pt) {
         LaunchShadeDebug(*v.dev, b, wc, p.integrator, w.n, p.intersect_mode, st);
         break;
@@ -188,7 +188,7 @@ extern "C" int muon_gpu_render_noalloc(MuonScene *scene, const MuonRenderParams 
       LaunchShadePath(*v.dev, w, sp, b, wc, k, w.n, st);
       if (slots > 0)
         LaunchOcclude(*v.dev, b, wc, k, slots, static_cast<int>(std::min<int64_t>(int64_t(w.n) * slots, INT32_MAX)),
-                      p.intersect_mode, stats_on, st);
+                      p.intersect_mode, stats_on, v.dev->num_nodes, st);
       LaunchFold(b, wc, k, slots, w.n, st);
       if (!bp.bounded) {
         uint32_t next = 0;  // host stack memory: no pinned allocation

@@ -1,0 +1,29 @@
+"""Variants of the traversal kernels against each other: which one runs is
+decided by the size of the scene or of the frame, and results must not depend
+on it."""
+import numpy as np
+import pytest
+
+import muon_gb300 as m
+from muon_gb300 import native, scenes
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [native.ISECT_EXACT, native.ISECT_FAST, native.ISECT_WATERTIGHT])
+@pytest.mark.parametrize("depth,rr", [(1, 0), (5, 0), (-1, 1)])
+def test_deep_tree_descent_changes_no_hits(lib, mode, depth, rr):
+    """The same primitives under a tree just below the size at which warps
+    leave the descent early, and one just above it (leaves of one primitive):
+    the same paths. Two primitives at exactly one distance may swap (at most
+    0.5% of rays in the hit fixtures, far fewer here), so all but 2% of the
+    pixels have to be equal to the bit."""
+    parsed = m.parse_string(scenes.dense_mesh(96, 64, 4, 5, level=4, clutter=4000, seed=4))
+    films = []
+    for leaf, above in ((0, False), (1, True)):
+        scene = m.Scene(parsed, max_leaf_size=leaf)
+        assert (scene.bvh()[0]["nodes"] >= 8192) == above
+        films.append(scene.render(intersect_mode=mode, max_depth=depth, russian_roulette=rr, seed=9))
+        scene.close()
+    a, b = films
+    assert np.array_equal(a.count, b.count)
+    assert (a.sum == b.sum).all(axis=-1).mean() >= 0.98
