@@ -27,3 +27,17 @@ def test_deep_tree_descent_changes_no_hits(lib, mode, depth, rr):
     a, b = films
     assert np.array_equal(a.count, b.count)
     assert (a.sum == b.sum).all(axis=-1).mean() >= 0.98
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width,height", [(1, 1), (5, 3), (152, 33), (61, 80)])
+@pytest.mark.parametrize("wave_paths", [31, 1000, 4865])
+def test_short_queues_trace_the_same_paths(lib, width, height, wave_paths):
+    """Queues of one ray to a few rays per warp, and around one ray for each
+    warp of a full grid (4,864 on 152 multiprocessors): the film does not
+    depend on how a frame is cut into wavefronts."""
+    scene = m.Scene.from_string(scenes.feature_mix(width, height, 2, "pathtracer", "mis", 6))
+    whole = scene.render(seed=3)
+    cut = scene.render(seed=3, wave_paths=min(wave_paths, 2 * width * height))
+    assert np.array_equal(whole.sum, cut.sum) and np.array_equal(whole.sum_sq, cut.sum_sq)
+    assert np.array_equal(whole.count, cut.count)
