@@ -347,8 +347,7 @@ constexpr int kRefillThreshold = MUON_REFILL_THRESHOLD;
 // (12,878), 12.20 / 11.43 (52,694), 13.39 / 12.44 (195,485); 1024x1024x16 84.2 /
 // 74.4 (773,807); there 8, 12 and 20 lanes give 78.1, 75.6 and 74.6. Shallow trees
 // lose, their lanes reach leaves together: sphere field (448 nodes) 1.99 / 2.17,
-// Cornell box 0.80 / 0.89; and so do batches of small trees (eight of 1,000 to
-// 10,000 triangles: 7.95 / 8.10 ms).
+// Cornell box 0.80 / 0.89. So do batches, whose wavefronts mix trees (batch.cc).
 constexpr int kDeepMinDescend = 16;
 constexpr int kDeepNodes = 8192;
 // Minimum resident blocks per SM the traversal kernels are compiled for.
@@ -485,104 +484,143 @@ __global__ void __launch_bounds__(kBlock, MUON_TRAVERSAL_MIN_BLOCKS) ExtendKerne
 }
 
 // ---- stable class partition (MUON_STABLE_CLASSES) ---------------------------------
-// Tile t holds queue entries [t * kClassTile, (t + 1) * kClassTile); its
-// class counts, then their exclusive prefix over tiles, live in the ints
-// after the class lists of b.order.
+// Two passes over the queue's classes, one block per segment of the queue: the
+// first leaves each segment's class counts in the ints after the class lists
+// of b.order, the second adds up the counts of all segments before its own,
+// and of the warps before each warp, and places its hits behind them. Warps
+// work on consecutive parts of a segment and keep their running positions in
+// registers, so the loops have no barriers. Bound by reading the classes and
+// writing the lists: 16.7 M entries take 92 us, 1.1 M 10 us (131 and 17 us with
+// a scan kernel between and three barriers per 256 entries); short queues by
+// the two launches, 9 us (13). Eight segments per SM: 4 and 16 are no faster.
 constexpr int kClassThreads = 256;
-static_assert(kClassTile % kClassThreads == 0, "a tile is a whole number of block passes");
+constexpr int kClassWarps = kClassThreads / 32;
+constexpr int kClassAhead = 4;  // class loads in flight per lane
+static_assert(kClassTile == kClassWarps * 32 * kClassAhead, "the smallest segment is one batch of loads");
 
 __device__ __forceinline__ int32_t *ClassTiles(const PathBuffers &b) {
   return b.order + static_cast<int64_t>(b.order_cap) * kNumClasses;
 }
 
+// Entries per segment: a multiple of kClassTile.
+__device__ __forceinline__ int ClassSegment(int n) {
+  const int segs = static_cast<int>(gridDim.x);
+  return ((n + segs - 1) / segs + kClassTile - 1) / kClassTile * kClassTile;
+}
+
+// The classes of entries j0 + 32 k + lane, -1 from `end` on.
+__device__ __forceinline__ void LoadClasses(const int32_t *link, int j0, int end, int lane, int (&c)[kClassAhead]) {
+#pragma unroll
+  for (int k = 0; k < kClassAhead; ++k) {
+    const int j = j0 + 32 * k + lane;
+    c[k] = j < end ? link[j] : -1;
+  }
+}
+
 __global__ void __launch_bounds__(kClassThreads) ClassCountKernel(PathBuffers b, WaveCounters wc, int bounce) {
   const int n = static_cast<int>(*wc.count(bounce));
-  const int base = blockIdx.x * kClassTile;
-  if (base >= n) return;
-  __shared__ int cnt[kNumClasses];
-  if (threadIdx.x < kNumClasses) cnt[threadIdx.x] = 0;
+  const int size = ClassSegment(n);
+  const int64_t begin = static_cast<int64_t>(blockIdx.x) * size;
+  if (begin >= n) return;
+  __shared__ int total[kNumClasses];
+  if (threadIdx.x < kNumClasses) total[threadIdx.x] = 0;
   __syncthreads();
-  for (int k = 0; k < kClassTile / kClassThreads; ++k) {
-    const int j = base + k * kClassThreads + threadIdx.x;
-    const int c = j < n ? b.link[j] : -1;
-    if (c >= 0 && c < kNumClasses) atomicAdd(&cnt[c], 1);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int end = static_cast<int>(min(static_cast<int64_t>(n), begin + size));
+  int cnt[kNumClasses] = {};
+  for (int j0 = static_cast<int>(begin) + 32 * kClassAhead * w; j0 < end; j0 += kClassTile) {
+    int c[kClassAhead];
+    LoadClasses(b.link, j0, end, lane, c);
+#pragma unroll
+    for (int k = 0; k < kClassAhead; ++k)
+#pragma unroll
+      for (int q = 0; q < kNumClasses; ++q) cnt[q] += c[k] == q ? 1 : 0;
+  }
+#pragma unroll
+  for (int q = 0; q < kNumClasses; ++q) {
+    cnt[q] = __reduce_add_sync(0xffffffffu, cnt[q]);
+    if (lane == 0 && cnt[q]) atomicAdd(&total[q], cnt[q]);
   }
   __syncthreads();
-  if (threadIdx.x < kNumClasses) ClassTiles(b)[blockIdx.x * 8 + threadIdx.x] = cnt[threadIdx.x];
+  if (threadIdx.x < kNumClasses) ClassTiles(b)[8 * blockIdx.x + threadIdx.x] = total[threadIdx.x];
 }
 
-// One block per class: the exclusive prefix of the class's tile counts, and
-// the class total for the shading kernel.
-__global__ void __launch_bounds__(1024) ClassScanKernel(PathBuffers b, WaveCounters wc, int bounce) {
-  const int n = static_cast<int>(*wc.count(bounce));
-  const int tiles = (n + kClassTile - 1) / kClassTile;
-  const int c = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int32_t *t8 = ClassTiles(b);
-  const int per = (tiles + 1023) / 1024;
-  const int t0 = threadIdx.x * per, t1 = min(t0 + per, tiles);
-  int sum = 0;
-  for (int t = t0; t < t1; ++t) sum += t8[t * 8 + c];
-  __shared__ int warp_sums[32];
-  int x = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) warp_sums[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    const int v = warp_sums[lane];
-    int y = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int z = __shfl_up_sync(0xffffffffu, y, o);
-      if (lane >= o) y += z;
-    }
-    warp_sums[lane] = y - v;  // exclusive over warps
-  }
-  __syncthreads();
-  int acc = warp_sums[w] + x - sum;
-  for (int t = t0; t < t1; ++t) {
-    const int v = t8[t * 8 + c];
-    t8[t * 8 + c] = acc;
-    acc += v;
-  }
-  if (threadIdx.x == 1023) wc.classes(bounce)[c] = static_cast<uint32_t>(acc);
-}
-
-// Each hit entry to its class list, in queue order.
+// Each hit entry to its class list, in queue order, and the class totals for
+// the shading kernel.
 __global__ void __launch_bounds__(kClassThreads) ClassScatterKernel(PathBuffers b, WaveCounters wc, int bounce) {
   const int n = static_cast<int>(*wc.count(bounce));
-  const int base = blockIdx.x * kClassTile;
-  if (base >= n) return;
-  constexpr int kW = kClassThreads / 32;
-  __shared__ int running[kNumClasses];
-  __shared__ int warp_cnt[kW][kNumClasses];
+  const int size = ClassSegment(n);
+  const int64_t begin64 = static_cast<int64_t>(blockIdx.x) * size;
+  if (begin64 >= n) return;
+  __shared__ int before[kNumClasses];             // hits in the segments before this one
+  __shared__ int warp_cnt[kClassWarps][kNumClasses];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x < kNumClasses) running[threadIdx.x] = ClassTiles(b)[blockIdx.x * 8 + threadIdx.x];
-  for (int k = 0; k < kClassTile / kClassThreads; ++k) {
-    const int j = base + k * kClassThreads + threadIdx.x;
-    int c = j < n ? b.link[j] : -1;
-    if (c >= kNumClasses) c = -1;
-    unsigned mine = 0;
+  if (threadIdx.x < kNumClasses) before[threadIdx.x] = 0;
+  __syncthreads();
+  // this warp's part of the segment
+  const int part = size / kClassWarps;
+  const int begin = static_cast<int>(begin64) + w * part;
+  const int end = min(n, begin + part);
+  int c[kClassAhead];
+  LoadClasses(b.link, begin, end, lane, c);
+  {
+    const int32_t *tiles = ClassTiles(b);
+    int sum[kNumClasses] = {};
+    for (int t = threadIdx.x; t < static_cast<int>(blockIdx.x); t += kClassThreads) {
+      const int2 *p = reinterpret_cast<const int2 *>(tiles + 8 * t);  // (24 bytes a path before it: 8-byte aligned)
+      const int2 c01 = p[0], c23 = p[1], c45 = p[2];
+      sum[0] += c01.x, sum[1] += c01.y, sum[2] += c23.x, sum[3] += c23.y, sum[4] += c45.x, sum[5] += c45.y;
+    }
+#pragma unroll
     for (int q = 0; q < kNumClasses; ++q) {
-      const unsigned m = __ballot_sync(0xffffffffu, c == q);
-      if (lane == 0) warp_cnt[w][q] = __popc(m);
-      if (c == q) mine = m;
+      sum[q] = __reduce_add_sync(0xffffffffu, sum[q]);
+      if (lane == 0 && sum[q]) atomicAdd(&before[q], sum[q]);
     }
-    __syncthreads();
-    if (c >= 0) {
-      int pos = running[c] + __popc(mine & ((1u << lane) - 1u));
-      for (int v = 0; v < w; ++v) pos += warp_cnt[v][c];
-      if (pos < b.order_cap) b.order[static_cast<int64_t>(c) * b.order_cap + pos] = j;
-    }
-    __syncthreads();
-    if (threadIdx.x < kNumClasses) {
-      int tot = 0;
-      for (int v = 0; v < kW; ++v) tot += warp_cnt[v][threadIdx.x];
-      running[threadIdx.x] += tot;
-    }
-    __syncthreads();
   }
+  int pos[kNumClasses] = {};
+  for (int j0 = begin; j0 < end; j0 += 32 * kClassAhead) {
+    int d[kClassAhead];
+    if (j0 == begin) {
+#pragma unroll
+      for (int k = 0; k < kClassAhead; ++k) d[k] = c[k];
+    } else {
+      LoadClasses(b.link, j0, end, lane, d);
+    }
+#pragma unroll
+    for (int k = 0; k < kClassAhead; ++k)
+#pragma unroll
+      for (int q = 0; q < kNumClasses; ++q) pos[q] += d[k] == q ? 1 : 0;
+  }
+#pragma unroll
+  for (int q = 0; q < kNumClasses; ++q) {
+    pos[q] = __reduce_add_sync(0xffffffffu, pos[q]);
+    if (lane == 0) warp_cnt[w][q] = pos[q];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kNumClasses; ++q) {
+    pos[q] = before[q];
+    for (int v = 0; v < w; ++v) pos[q] += warp_cnt[v][q];
+  }
+  const unsigned below = (1u << lane) - 1u;
+  for (int j0 = begin; j0 < end; j0 += 32 * kClassAhead) {
+    if (j0 != begin) LoadClasses(b.link, j0, end, lane, c);
+#pragma unroll
+    for (int k = 0; k < kClassAhead; ++k) {
+      int at = -1;
+#pragma unroll
+      for (int q = 0; q < kNumClasses; ++q) {
+        const unsigned m = __ballot_sync(0xffffffffu, c[k] == q);
+        if (c[k] == q) at = pos[q] + __popc(m & below);
+        pos[q] += __popc(m);
+      }
+      if (at >= 0 && at < b.order_cap) b.order[static_cast<int64_t>(c[k]) * b.order_cap + at] = j0 + 32 * k + lane;
+    }
+  }
+  // the last segment's last warp ends at the class totals
+  if (begin64 + size >= n && w == kClassWarps - 1 && lane == 0)
+#pragma unroll
+    for (int q = 0; q < kNumClasses; ++q) wc.classes(bounce)[q] = static_cast<uint32_t>(pos[q]);
 }
 
 // Shadow queue entries are slot indices (entry * S + slot). A blocked slot's
@@ -1578,7 +1616,7 @@ void LaunchCamera(const DevCamera &cam, const WaveInfo &w, const PathBuffers &b,
 }
 
 void LaunchExtend(const DevScene &s, const PathBuffers &b, WaveCounters wc, int bounce, int bound, int isect,
-                  bool stats, int tree_nodes, cudaStream_t st) {
+                  bool stats, int tree_nodes, bool classes, cudaStream_t st) {
   if (bound <= 0) return;
   WithMode(isect, [&](auto m) {
     constexpr int M = decltype(m)::value;
@@ -1587,11 +1625,11 @@ void LaunchExtend(const DevScene &s, const PathBuffers &b, WaveCounters wc, int 
     else if (tree_nodes >= kDeepNodes) ExtendKernel<false, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
     else ExtendKernel<false, M, false><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
   });
-  if (MUON_STABLE_CLASSES) {
-    const unsigned tiles = static_cast<unsigned>((bound + kClassTile - 1) / kClassTile);
-    ClassCountKernel<<<tiles, kClassThreads, 0, st>>>(b, wc, bounce);
-    ClassScanKernel<<<kNumClasses, 1024, 0, st>>>(b, wc, bounce);
-    ClassScatterKernel<<<tiles, kClassThreads, 0, st>>>(b, wc, bounce);
+  if (MUON_STABLE_CLASSES && classes) {
+    const int64_t segs = (static_cast<int64_t>(bound) + kClassTile - 1) / kClassTile;
+    const unsigned g = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(segs, 8 * g_sms)));
+    ClassCountKernel<<<g, kClassThreads, 0, st>>>(b, wc, bounce);
+    ClassScatterKernel<<<g, kClassThreads, 0, st>>>(b, wc, bounce);
   }
 }
 

@@ -86,8 +86,9 @@ struct PathBuffers {
 };
 
 // The `order` array of a wavefront of `cap` paths: kNumClasses class lists
-// of cap entries each, then 8 class counts per tile of kClassTile queue
-// entries (the stable class partition's, MUON_STABLE_CLASSES in kernels.cu).
+// of cap entries each, then 8 class counts per segment of at least kClassTile
+// queue entries (the stable class partition's, MUON_STABLE_CLASSES in
+// kernels.cu).
 constexpr int kClassTile = 1024;
 inline int64_t OrderInts(int64_t cap) { return cap * kNumClasses + (cap / kClassTile + 1) * 8; }
 
@@ -134,10 +135,11 @@ void SetPersistentGrid(int blocks);
 void SetTraversalGrid(int sms);
 
 void LaunchCamera(const DevCamera &cam, const WaveInfo &w, const PathBuffers &b, WaveCounters wc, cudaStream_t st);
-// tree_nodes: nodes of one scene's BVH (the mean over a batch), which picks the
-// traversal kernels' variant.
+// tree_nodes: nodes of the scene's BVH, which picks the traversal kernels'
+// variant (0 for a batch). classes: build the class lists (which the path
+// tracer's shading reads and the preview integrators' does not).
 void LaunchExtend(const DevScene &s, const PathBuffers &b, WaveCounters wc, int bounce, int bound, int isect,
-                  bool stats, int tree_nodes, cudaStream_t st);
+                  bool stats, int tree_nodes, bool classes, cudaStream_t st);
 void LaunchShadeDebug(const DevScene &s, const PathBuffers &b, WaveCounters wc, int integrator, int bound, int isect,
                       cudaStream_t st);
 // Raytracer / AnalyticDirect for every path of a wave; rays are traced up to

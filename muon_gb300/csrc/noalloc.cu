@@ -180,7 +180,7 @@ extern "C" int muon_gpu_render_noalloc(MuonScene *scene, const MuonRenderParams 
     WaveCounters wc{counters};
     LaunchCamera(*v.cam, w, b, wc, st);
     for (int k = 0; k < bp.bounces; ++k) {
-      LaunchExtend(*v.dev, b, wc, k, w.n, p.intersect_mode, stats_on, v.dev->num_nodes, st);
+      LaunchExtend(*v.dev, b, wc, k, w.n, p.intersect_mode, stats_on, v.dev->num_nodes, pt, st);
       if (!pt) {
         LaunchShadeDebug(*v.dev, b, wc, p.integrator, w.n, p.intersect_mode, st);
         break;

@@ -672,7 +672,7 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
       }
       for (int k = 0; k < (whitted ? 0 : bounces); ++k) {
         sample_queue(wi, wc, k, 0);
-        timed(0, [&] { LaunchExtend(sc->dev, b, wc, k, w.n, p.intersect_mode, stats_on, sc->dev.num_nodes, st); });
+        timed(0, [&] { LaunchExtend(sc->dev, b, wc, k, w.n, p.intersect_mode, stats_on, sc->dev.num_nodes, pt, st); });
         // Guiding covers the first rec_bounces vertices of a path (where the
         // network is trained); deeper vertices sample the BRDF alone.
         const bool guided = guide && k < guide->rec_bounces;

@@ -41,3 +41,19 @@ def test_short_queues_trace_the_same_paths(lib, width, height, wave_paths):
     cut = scene.render(seed=3, wave_paths=min(wave_paths, 2 * width * height))
     assert np.array_equal(whole.sum, cut.sum) and np.array_equal(whole.sum_sq, cut.sum_sq)
     assert np.array_equal(whole.count, cut.count)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width,height,paths", [(61, 47, 31), (61, 47, 1023), (61, 47, 1024), (61, 47, 1025),
+                                                (96, 64, 4096 + 129), (1301, 1010, 1216 * 1024 - 1),
+                                                (1301, 1010, 1216 * 1024 + 1), (1301, 1010, 1301 * 1010)])
+def test_class_lists_hold_every_hit(lib, width, height, paths):
+    """The stable class partition at the edges of its segments (1,024 entries,
+    and one segment per block of a full grid, 1,216 on 152 multiprocessors):
+    hits missing from a list, or in it twice, would change the film. Wavefronts
+    of `paths` paths against wavefronts of another size."""
+    scene = m.Scene.from_string(scenes.feature_mix(width, height, 1, "pathtracer", "mis", 3))
+    film = scene.render(seed=2, wave_paths=paths)
+    other = scene.render(seed=2, wave_paths=700 if width < 100 else 262144)
+    assert np.array_equal(film.sum, other.sum) and np.array_equal(film.count, other.count)
+    assert (film.sum > 0).mean() > 0.2
