@@ -39,7 +39,7 @@ constexpr int kMaxEventPairs = 16384;
 
 // The path arrays of one wavefront in flight (PathBuffers).
 struct WorkSet {
-  DeviceBuffer ray_o[2], ray_d[2], tp[2], rad[2], hits, link, final_rad, org, contrib, slot_dir, shq, order;
+  DeviceBuffer ray_o[2], ray_d[2], tp[2], rad[2], hits[2], link[2], final_rad, org, contrib, slot_dir, shq, order;
   int64_t cap = 0;
   int slots = -1;
 
@@ -53,9 +53,9 @@ struct WorkSet {
       EnsurePooled(ray_d[k], p * sizeof(float4), device);
       EnsurePooled(tp[k], p * sizeof(float4), device);
       EnsurePooled(rad[k], p * sizeof(float4), device);
+      EnsurePooled(hits[k], p * sizeof(int2), device);
+      EnsurePooled(link[k], p * sizeof(int32_t), device);
     }
-    EnsurePooled(hits, p * sizeof(int2), device);
-    EnsurePooled(link, p * sizeof(int32_t), device);
     EnsurePooled(final_rad, p * sizeof(float4), device);
     EnsurePooled(org, p * sizeof(float4), device);
     const size_t sl = static_cast<size_t>(p) * std::max(sl_count, 1);
@@ -68,7 +68,10 @@ struct WorkSet {
     return true;
   }
 
-  PathBuffers Buffers(const DeviceBuffer &stats) const {
+  // The arrays as bounce `bounce` uses them: hits and links alternate, so that
+  // a bounce's fold may still read its own while the next bounce's rays are
+  // traced.
+  PathBuffers Buffers(const DeviceBuffer &stats, int bounce) const {
     PathBuffers b;
     for (int k = 0; k < 2; ++k) {
       b.ray_o[k] = ray_o[k].as<float4>();
@@ -76,8 +79,8 @@ struct WorkSet {
       b.tp[k] = tp[k].as<float4>();
       b.rad[k] = rad[k].as<float4>();
     }
-    b.hits = hits.as<int2>();
-    b.link = link.as<int32_t>();
+    b.hits = hits[bounce & 1].as<int2>();
+    b.link = link[bounce & 1].as<int32_t>();
     b.final_rad = final_rad.as<float4>();
     b.org = org.as<float4>();
     b.contrib = contrib.as<float4>();
@@ -96,8 +99,10 @@ struct WorkSet {
       PoolGive(ray_d[k], device);
       PoolGive(tp[k], device);
       PoolGive(rad[k], device);
+      PoolGive(hits[k], device);
+      PoolGive(link[k], device);
     }
-    for (DeviceBuffer *b : {&hits, &link, &final_rad, &org, &contrib, &slot_dir, &shq, &order}) PoolGive(*b, device);
+    for (DeviceBuffer *b : {&final_rad, &org, &contrib, &slot_dir, &shq, &order}) PoolGive(*b, device);
   }
 };
 
@@ -107,6 +112,11 @@ struct MuonScene {
   // A second stream and its events, for wavefronts in flight two at a time.
   cudaStream_t stream2 = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr, film_ev[2] = {nullptr, nullptr};
+  // Per wavefront in flight: a stream for the next bounce's rays, and the events
+  // that fork it from the wavefront's own and join it.
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t shade_ev[2] = {nullptr, nullptr}, extend_ev[2] = {nullptr, nullptr};
+  cudaEvent_t count_ev[2][2] = {};  // per wavefront in flight: queue lengths read back (unbounded depth)
   SceneImage img;
   // The leaf-order records of a scene whose BVH was built on the device live
   // on the device only (img holds them in input order) until a host reader
@@ -142,14 +152,18 @@ struct MuonScene {
   ~MuonScene() {
     // The work arrays go to the process-wide cache once the stream is idle.
     if (stream && cudaStreamSynchronize(stream) == cudaSuccess &&
-        (!stream2 || cudaStreamSynchronize(stream2) == cudaSuccess)) {
+        (!stream2 || cudaStreamSynchronize(stream2) == cudaSuccess) &&
+        (!side[0] || cudaStreamSynchronize(side[0]) == cudaSuccess) &&
+        (!side[1] || cudaStreamSynchronize(side[1]) == cudaSuccess)) {
       for (WorkSet &ws : work) ws.Give(device);
       for (DeviceBuffer *b : {&film_sum, &film_sq, &film_cnt, &nodes, &prims, &prims_obj, &shade, &smooth, &smooth_obj})
         PoolGive(*b, device);
     }
-    for (cudaEvent_t e : {fork_ev, join_ev, film_ev[0], film_ev[1]})
+    for (cudaEvent_t e : {fork_ev, join_ev, film_ev[0], film_ev[1], count_ev[0][0], count_ev[0][1], count_ev[1][0],
+                          count_ev[1][1], shade_ev[0], shade_ev[1], extend_ev[0], extend_ev[1]})
       if (e) cudaEventDestroy(e);
-    if (stream2) cudaStreamDestroy(stream2);
+    for (cudaStream_t s : {stream2, side[0], side[1]})
+      if (s) cudaStreamDestroy(s);
     if (graph) cudaGraphExecDestroy(graph);
     for (EventPair &e : events) {
       if (e.a) cudaEventDestroy(e.a);
@@ -172,7 +186,7 @@ struct MuonScene {
     return e;
   }
 
-  PathBuffers Buffers(int set = 0) const { return work[set].Buffers(stats); }
+  PathBuffers Buffers(int set, int bounce) const { return work[set].Buffers(stats, bounce); }
 
   // Grows the path arrays of `sets` wavefronts in flight; true if any moved.
   bool EnsureWork(int64_t paths, int slots, int sets = 1) {
@@ -185,8 +199,19 @@ struct MuonScene {
   void EnsureStream2() {
     if (stream2) return;
     CUDA_TRY(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
-    for (cudaEvent_t *e : {&fork_ev, &join_ev, &film_ev[0], &film_ev[1]})
+    for (cudaEvent_t *e : {&fork_ev, &join_ev, &film_ev[0], &film_ev[1], &count_ev[0][0], &count_ev[0][1],
+                           &count_ev[1][0], &count_ev[1][1]})
       CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  }
+
+  // The side streams of `sets` wavefronts in flight and their events.
+  void EnsureSide(int sets) {
+    for (int k = 0; k < sets; ++k) {
+      if (side[k]) continue;
+      CUDA_TRY(cudaEventCreateWithFlags(&shade_ev[k], cudaEventDisableTiming));
+      CUDA_TRY(cudaEventCreateWithFlags(&extend_ev[k], cudaEventDisableTiming));
+      CUDA_TRY(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
+    }
   }
 
   // Grows the device and pinned host counter arrays; returns true if the
@@ -599,9 +624,6 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   // Keep per-wave path state within ~8 GiB.
   budget = std::max<int64_t>(1, std::min<int64_t>(budget, (int64_t(8) << 30) / WorkBytesPerPath(slots)));
   budget = std::min<int64_t>(budget, kMaxWavePaths);
-  const WavePlan plan = PlanWaves(W, H, p, budget);
-  std::vector<WaveInfo> waves(plan.Count());
-  for (size_t i = 0; i < waves.size(); ++i) waves[i] = plan.At(i);
   const BouncePlan bp = PlanBounces(p, sp);
   const bool traces = bp.traces, bounded = bp.bounded;
   const int bounces = bp.bounces;
@@ -609,15 +631,26 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   // Two wavefronts in flight, on two streams with their own path arrays:
   // while one wavefront's kernels drain (the last rays of a persistent
   // traversal launch, the last blocks of a pass), the other's fill the SMs.
-  // Films are still added in wave order. Per-kernel timing, probes, guiding
-  // and host-driven unbounded loops run the wavefronts one after another.
-  const bool concurrent = MUON_WAVES_IN_FLIGHT > 1 && bounded && !timing && !probe && !guide && waves.size() > 1;
+  // Films are still added in wave order. Per-kernel timing, probes and guiding
+  // run the wavefronts one after another.
+  const bool in_pairs = MUON_WAVES_IN_FLIGHT > 1 && !timing && !probe && !guide && (bounded || pt);
+  const WavePlan plan = PlanWaves(W, H, p, budget);
+  std::vector<WaveInfo> waves(plan.Count());
+  for (size_t i = 0; i < waves.size(); ++i) waves[i] = plan.At(i);
+  const bool concurrent = in_pairs && waves.size() > 1;
   bool moved = sc->EnsureWork(std::min<int64_t>(plan.pix_per_wave, npix_total) * plan.ns, slots, concurrent ? 2 : 1);
   moved |= sc->EnsureCounters(stride * waves.size());
   sc->stats.Ensure(sizeof(unsigned long long) * kNumStats);
-  if (concurrent) sc->EnsureStream2();
-  const PathBuffers bsets[2] = {sc->Buffers(0), sc->Buffers(concurrent ? 1 : 0)};
-  const PathBuffers &b = bsets[0];
+  if (concurrent || !bounded) sc->EnsureStream2();
+  const int last_set = concurrent ? 1 : 0;
+  const PathBuffers bsets[2][2] = {{sc->Buffers(0, 0), sc->Buffers(0, 1)},
+                                   {sc->Buffers(last_set, 0), sc->Buffers(last_set, 1)}};
+  // The next bounce's rays are traced beside a bounce's shadow rays and fold:
+  // both follow from its shading, and where one's queue runs out the other
+  // fills the chip (or, with short queues, hides its latency).
+  const bool lagged = !bounded && in_pairs;
+  const bool overlap = pt && bounces > 1 && !timing && !probe && (bounded || lagged);
+  if (overlap) sc->EnsureSide(last_set + 1);
   if (probe) {
     probe->waves = waves.size();
     probe->bounces = bounces;
@@ -627,7 +660,7 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   }
   auto sample_queue = [&](size_t wi, WaveCounters wc, int k, int kind) {
     if (probe)
-      LaunchSampleQueue(b, wc, k, kind, slots, probe->m, probe->buf.as<float4>() + probe->Offset(wi, k, kind), st);
+      LaunchSampleQueue(bsets[0][k & 1], wc, k, kind, slots, probe->m, probe->buf.as<float4>() + probe->Offset(wi, k, kind), st);
   };
 
   uint64_t launches = 0;
@@ -643,78 +676,147 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
       CUDA_TRY(cudaEventRecord(sc->fork_ev, main_st));
       CUDA_TRY(cudaStreamWaitEvent(sc->stream2, sc->fork_ev, 0));
     }
-    for (size_t wi = 0; wi < waves.size(); ++wi) {
-      const WaveInfo &w = waves[wi];
-      WaveCounters wc{sc->counters.as<uint32_t>() + wi * stride};
-      // this wavefront's path arrays and stream
-      const int set = concurrent ? static_cast<int>(wi & 1) : 0;
-      const PathBuffers &b = bsets[set];
-      const cudaStream_t st = set ? sc->stream2 : main_st;
-      LaunchCamera(sc->cam, w, b, wc, st);
+    // Wavefront wi's path arrays and stream.
+    auto set_of = [&](size_t wi) { return concurrent ? static_cast<int>(wi & 1) : 0; };
+    auto stream_of = [&](size_t wi) { return set_of(wi) ? sc->stream2 : main_st; };
+    auto counters_of = [&](size_t wi) { return WaveCounters{sc->counters.as<uint32_t>() + wi * stride}; };
+    auto timed = [&](int kind, cudaStream_t st, auto &&launch) {
+      // External event nodes when captured, so they time the kernels
+      // inside the replayed graph.
+      EventPair *ev = timing ? sc->NextEvent(kind) : nullptr;
+      if (ev) CUDA_TRY(capturing ? cudaEventRecordWithFlags(ev->a, st, cudaEventRecordExternal)
+                                 : cudaEventRecord(ev->a, st));
+      launch();
+      if (ev) CUDA_TRY(capturing ? cudaEventRecordWithFlags(ev->b, st, cudaEventRecordExternal)
+                                 : cudaEventRecord(ev->b, st));
       ++launches;
-      auto timed = [&](int kind, auto &&launch) {
-        // External event nodes when captured, so they time the kernels
-        // inside the replayed graph.
-        EventPair *ev = timing ? sc->NextEvent(kind) : nullptr;
-        if (ev) CUDA_TRY(capturing ? cudaEventRecordWithFlags(ev->a, st, cudaEventRecordExternal)
-                                   : cudaEventRecord(ev->a, st));
-        launch();
-        if (ev) CUDA_TRY(capturing ? cudaEventRecordWithFlags(ev->b, st, cudaEventRecordExternal)
-                                   : cudaEventRecord(ev->b, st));
-        ++launches;
-      };
+    };
+    // Camera rays of a wavefront (and the whole of it for the integrators that
+    // follow each path to its end in one launch).
+    auto begin_wave = [&](size_t wi) {
+      const WaveInfo &w = waves[wi];
+      const PathBuffers &b = bsets[set_of(wi)][0];
+      const cudaStream_t st = stream_of(wi);
+      LaunchCamera(sc->cam, w, b, counters_of(wi), st);
+      ++launches;
       if (whitted && bounces > 0) {
         // Integrator::Trace's depth cut-off; unbounded depth stops at the
         // bounce cap (a ray between two mirrors would never end).
         const int max_d = p.integrator == MUON_INTEGRATOR_ANALYTIC_DIRECT ? 0
                           : sp.max_trace_depth >= 0 ? sp.max_trace_depth : kMaxBounces - 1;
-        timed(2, [&] { LaunchWhitted(sc->dev, b, w, p.integrator, max_d, p.intersect_mode, stats_on, st); });
+        timed(2, st, [&] { LaunchWhitted(sc->dev, b, w, p.integrator, max_d, p.intersect_mode, stats_on, st); });
       }
-      for (int k = 0; k < (whitted ? 0 : bounces); ++k) {
-        sample_queue(wi, wc, k, 0);
-        timed(0, [&] { LaunchExtend(sc->dev, b, wc, k, w.n, p.intersect_mode, stats_on, sc->dev.num_nodes, pt, st); });
-        // Guiding covers the first rec_bounces vertices of a path (where the
-        // network is trained); deeper vertices sample the BRDF alone.
-        const bool guided = guide && k < guide->rec_bounces;
-        if (guided) {
-          // two kernels: the features, then the tensor-core network pass
-          timed(2, [&] { LaunchGuideInfer(sc->dev, b, wc, k, w.n, p.intersect_mode, guide_local, st); });
-          ++launches;
-        }
-        if (!pt) {
-          timed(2, [&] { LaunchShadeDebug(sc->dev, b, wc, p.integrator, w.n, p.intersect_mode, st); });
-          break;
-        }
-        timed(2, [&] {
-          if (guided) LaunchShadePathGuided(sc->dev, w, sp, b, wc, k, w.n, guide_local, st);
-          else LaunchShadePath(sc->dev, w, sp, b, wc, k, w.n, st);
-        });
-        if (slots > 0) {
-          sample_queue(wi, wc, k, 1);
-          timed(1, [&] {
-            LaunchOcclude(sc->dev, b, wc, k, slots, static_cast<int>(std::min<int64_t>(int64_t(w.n) * slots, INT32_MAX)),
-                          p.intersect_mode, stats_on, sc->dev.num_nodes, st);
-          });
-        }
-        timed(3, [&] {
-          if (guided) LaunchFoldGuided(b, wc, k, slots, w.n, guide_local, st);
-          else LaunchFold(b, wc, k, slots, w.n, st);
-        });
-        if (guided) launches += 2;  // the ordered append of training samples
-        if (host_loop) {
-          CUDA_TRY(cudaMemcpyAsync(sc->h_counters, wc.count(k + 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-          CUDA_TRY(cudaStreamSynchronize(st));
-          if (sc->h_counters[0] == 0) break;
-        }
+    };
+    // Closest hits and class lists of bounce k.
+    auto trace = [&](size_t wi, int k, cudaStream_t st) {
+      const WaveInfo &w = waves[wi];
+      const PathBuffers &b = bsets[set_of(wi)][k & 1];
+      sample_queue(wi, counters_of(wi), k, 0);
+      timed(0, st, [&] {
+        LaunchExtend(sc->dev, b, counters_of(wi), k, w.n, p.intersect_mode, stats_on, sc->dev.num_nodes, pt, st);
+      });
+    };
+    auto bounce = [&](size_t wi, int k) {
+      const WaveInfo &w = waves[wi];
+      const WaveCounters wc = counters_of(wi);
+      const int set = set_of(wi);
+      const PathBuffers &b = bsets[set][k & 1];
+      const cudaStream_t st = stream_of(wi);
+      if (!overlap || k == 0) trace(wi, k, st);
+      // Guiding covers the first rec_bounces vertices of a path (where the
+      // network is trained); deeper vertices sample the BRDF alone.
+      const bool guided = guide && k < guide->rec_bounces;
+      if (guided) {
+        // two kernels: the features, then the tensor-core network pass
+        timed(2, st, [&] { LaunchGuideInfer(sc->dev, b, wc, k, w.n, p.intersect_mode, guide_local, st); });
+        ++launches;
       }
+      if (!pt) {
+        timed(2, st, [&] { LaunchShadeDebug(sc->dev, b, wc, p.integrator, w.n, p.intersect_mode, st); });
+        return;
+      }
+      timed(2, st, [&] {
+        if (guided) LaunchShadePathGuided(sc->dev, w, sp, b, wc, k, w.n, guide_local, st);
+        else LaunchShadePath(sc->dev, w, sp, b, wc, k, w.n, st);
+      });
+      const bool ahead = overlap && k + 1 < bounces;
+      if (ahead) {
+        CUDA_TRY(cudaEventRecord(sc->shade_ev[set], st));
+        CUDA_TRY(cudaStreamWaitEvent(sc->side[set], sc->shade_ev[set], 0));
+        trace(wi, k + 1, sc->side[set]);
+        CUDA_TRY(cudaEventRecord(sc->extend_ev[set], sc->side[set]));
+      }
+      if (slots > 0) {
+        sample_queue(wi, wc, k, 1);
+        timed(1, st, [&] {
+          LaunchOcclude(sc->dev, b, wc, k, slots, static_cast<int>(std::min<int64_t>(int64_t(w.n) * slots, INT32_MAX)),
+                        p.intersect_mode, stats_on, sc->dev.num_nodes, st);
+        });
+      }
+      timed(3, st, [&] {
+        if (guided) LaunchFoldGuided(b, wc, k, slots, w.n, guide_local, st);
+        else LaunchFold(b, wc, k, slots, w.n, st);
+      });
+      if (guided) launches += 2;  // the ordered append of training samples
+      if (ahead) CUDA_TRY(cudaStreamWaitEvent(st, sc->extend_ev[set], 0));
+    };
+    auto end_wave = [&](size_t wi) {
+      const PathBuffers &b = bsets[set_of(wi)][0];
+      const cudaStream_t st = stream_of(wi);
       // films in wave order (wavefronts may share pixels)
       if (concurrent && wi > 0) CUDA_TRY(cudaStreamWaitEvent(st, sc->film_ev[(wi - 1) & 1], 0));
-      LaunchFilm(w, b, d_sum, d_sq, d_cnt, st);
+      LaunchFilm(waves[wi], b, d_sum, d_sq, d_cnt, st);
       if (concurrent) CUDA_TRY(cudaEventRecord(sc->film_ev[wi & 1], st));
       ++launches;
       if (guide && !guide->direct_only) {
-        LaunchGuideCollect(b, wc, std::min(bounces, guide->rec_bounces), w.n, guide_local, st);
+        LaunchGuideCollect(b, counters_of(wi), std::min(bounces, guide->rec_bounces), waves[wi].n, guide_local, st);
         ++launches;
+      }
+    };
+    const int wave_bounces = whitted ? 0 : bounces;
+    if (host_loop && lagged) {
+      // One or two wavefronts at a time, bounce by bounce. The host learns of a
+      // queue's length while the next bounce already runs: a wavefront ends
+      // with one bounce that finds no path.
+      for (size_t first = 0; first < waves.size(); first += 2) {
+        const size_t last = std::min(waves.size(), first + 2);
+        bool on[2] = {false, false};
+        for (size_t wi = first; wi < last; ++wi) begin_wave(wi), on[wi & 1] = true;
+        for (int k = 0; k < wave_bounces && (on[0] || on[1]); ++k) {
+          for (size_t wi = first; wi < last; ++wi) {
+            const int s = static_cast<int>(wi & 1);
+            if (!on[s]) continue;
+            uint32_t *h = sc->h_counters + wi * stride;  // word 16 k: paths at bounce k
+            if (k >= 2) {
+              CUDA_TRY(cudaEventSynchronize(sc->count_ev[s][k & 1]));  // recorded at bounce k - 2
+              if (h[16 * (k - 1)] == 0) {
+                on[s] = false;
+                continue;
+              }
+            }
+            bounce(wi, k);
+            const WaveCounters wc = counters_of(wi);
+            CUDA_TRY(cudaMemcpyAsync(h + 16 * (k + 1), wc.count(k + 1), sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                     stream_of(wi)));
+            CUDA_TRY(cudaEventRecord(sc->count_ev[s][k & 1], stream_of(wi)));
+          }
+        }
+        for (size_t wi = first; wi < last; ++wi) end_wave(wi);
+      }
+    } else {
+      for (size_t wi = 0; wi < waves.size(); ++wi) {
+        begin_wave(wi);
+        for (int k = 0; k < wave_bounces; ++k) {
+          bounce(wi, k);
+          if (!pt) break;
+          if (host_loop) {
+            CUDA_TRY(cudaMemcpyAsync(sc->h_counters, counters_of(wi).count(k + 1), sizeof(uint32_t),
+                                     cudaMemcpyDeviceToHost, st));
+            CUDA_TRY(cudaStreamSynchronize(st));
+            if (sc->h_counters[0] == 0) break;
+          }
+        }
+        end_wave(wi);
       }
     }
     if (concurrent) {  // the second stream's work ends before the frame does

@@ -57,3 +57,23 @@ def test_class_lists_hold_every_hit(lib, width, height, paths):
     other = scene.render(seed=2, wave_paths=700 if width < 100 else 262144)
     assert np.array_equal(film.sum, other.sum) and np.array_equal(film.count, other.count)
     assert (film.sum > 0).mean() > 0.2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width,height,spp,depth,nee", [(1, 1, 1, 2, "mis"), (33, 31, 3, 1, "mis"), (129, 127, 7, 5, "off"),
+                                                        (129, 127, 7, -1, "mis"), (181, 183, 2, -1, "on")])
+def test_overlapped_bounces_render_the_same_film(lib, width, height, spp, depth, nee):
+    """Bounces whose next rays are traced beside their shadow rays and fold, in
+    one wavefront and in two or three at a time, against kernels run one after
+    another (a render with per-kernel timing): bit for bit the same film, also
+    when the frame is replayed."""
+    scene = m.Scene.from_string(scenes.feature_mix(width, height, spp, "pathtracer", "mis", 5))
+    kw = dict(seed=6, max_depth=depth, russian_roulette=1 if depth < 0 else 0, next_event_estimation=nee)
+    serial = scene.render(flags=native.RENDER_TIMING, **kw)
+    paths = width * height * spp
+    for wave_paths in (0, (paths + 1) // 2, (paths + 2) // 3):
+        for _ in range(3):
+            film = scene.render(wave_paths=wave_paths, **kw)
+            assert np.array_equal(film.sum, serial.sum) and np.array_equal(film.sum_sq, serial.sum_sq)
+            assert np.array_equal(film.count, serial.count)
+    assert scene.stats()["paths"] == paths
