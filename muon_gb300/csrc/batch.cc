@@ -57,8 +57,8 @@ struct MuonBatch {
   std::vector<uint64_t> scene_prims;
   uint64_t total_nodes = 0, total_prims = 0;
   // work
-  DeviceBuffer ray_o[2], ray_d[2], tp[2], rad[2], hits, link, final_rad, org, contrib, slot_dir, shq, order, counters,
-      stats, scene_table, seg_table;
+  DeviceBuffer ray_o[2], ray_d[2], tp[2], rad[2], hits[2], link[2], final_rad, org, contrib, slot_dir, shq, order,
+      counters, stats, scene_table, seg_table;
   std::vector<DeviceBuffer> film_sum, film_sq, film_cnt;
   int64_t wave_cap = 0;
   int slots_cap = -1;
@@ -68,6 +68,9 @@ struct MuonBatch {
   uint64_t graph_launches = 0;
   std::vector<cudaEvent_t> wave_done;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
+  // the next bounce's rays beside a bounce's shadow rays and fold (render.cc)
+  cudaStream_t side = nullptr;
+  cudaEvent_t shade_ev = nullptr, extend_ev = nullptr;
   // launch configuration
   int wave_paths = 0;       // 0: default
   int blocks_per_sm = 0;    // 0: default traversal grid
@@ -80,6 +83,9 @@ struct MuonBatch {
     for (cudaEvent_t e : wave_done) cudaEventDestroy(e);
     if (t0) cudaEventDestroy(t0);
     if (t1) cudaEventDestroy(t1);
+    if (shade_ev) cudaEventDestroy(shade_ev);
+    if (extend_ev) cudaEventDestroy(extend_ev);
+    if (side) cudaStreamDestroy(side);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -89,7 +95,8 @@ struct MuonBatch {
     graph_key.clear();
   }
 
-  PathBuffers Buffers() const {
+  // As bounce `bounce` uses them: hits and links alternate (WorkSet in render.cc).
+  PathBuffers Buffers(int bounce) const {
     PathBuffers b;
     for (int k = 0; k < 2; ++k) {
       b.ray_o[k] = ray_o[k].as<float4>();
@@ -97,8 +104,8 @@ struct MuonBatch {
       b.tp[k] = tp[k].as<float4>();
       b.rad[k] = rad[k].as<float4>();
     }
-    b.hits = hits.as<int2>();
-    b.link = link.as<int32_t>();
+    b.hits = hits[bounce & 1].as<int2>();
+    b.link = link[bounce & 1].as<int32_t>();
     b.final_rad = final_rad.as<float4>();
     b.org = org.as<float4>();
     b.contrib = contrib.as<float4>();
@@ -119,9 +126,9 @@ struct MuonBatch {
       ray_d[k].Ensure(p * sizeof(float4));
       tp[k].Ensure(p * sizeof(float4));
       rad[k].Ensure(p * sizeof(float4));
+      hits[k].Ensure(p * sizeof(int2));
+      link[k].Ensure(p * sizeof(int32_t));
     }
-    hits.Ensure(p * sizeof(int2));
-    link.Ensure(p * sizeof(int32_t));
     final_rad.Ensure(p * sizeof(float4));
     org.Ensure(p * sizeof(float4));
     size_t sl = static_cast<size_t>(p) * std::max(s, 1);
@@ -348,7 +355,12 @@ void RenderBatch(MuonBatch *b, const MuonRenderParams *params, double *const *d_
   if (!b->t0) CUDA_TRY(cudaEventCreate(&b->t0));
   if (!b->t1) CUDA_TRY(cudaEventCreate(&b->t1));
 
-  PathBuffers pb = b->Buffers();
+  if (!b->side) {
+    CUDA_TRY(cudaEventCreateWithFlags(&b->shade_ev, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventCreateWithFlags(&b->extend_ev, cudaEventDisableTiming));
+    CUDA_TRY(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
+  }
+  const PathBuffers pbs[2] = {b->Buffers(0), b->Buffers(1)};
   const BatchScene *d_scenes = b->scene_table.as<BatchScene>();
   const BatchSeg *d_segs = b->seg_table.as<BatchSeg>();
   uint64_t launches = 0;
@@ -363,12 +375,24 @@ void RenderBatch(MuonBatch *b, const MuonRenderParams *params, double *const *d_
       const WavePlan &w = waves[wi];
       WaveCounters wc{b->counters.as<uint32_t>() + wi * stride};
       const BatchSeg *wsegs = d_segs + w.seg_begin;
-      LaunchCameraBatch(d_scenes, wsegs, w.nseg, w.paths, pb, wc, st);
+      LaunchCameraBatch(d_scenes, wsegs, w.nseg, w.paths, pbs[0], wc, st);
       ++launches;
+      auto trace = [&](int k, cudaStream_t on) {
+        LaunchExtend(b->dev, pbs[k & 1], wc, k, w.paths, isect, stats_on, tree_nodes, true, on);
+        ++launches;
+      };
+      if (w.bounces > 0) trace(0, st);
       for (int k = 0; k < w.bounces; ++k) {
-        LaunchExtend(b->dev, pb, wc, k, w.paths, isect, stats_on, tree_nodes, true, st);
+        const PathBuffers &pb = pbs[k & 1];
         LaunchShadePathBatch(b->dev, d_scenes, wsegs, S, isect, pb, wc, k, w.paths, st);
-        launches += 2;
+        ++launches;
+        const bool ahead = k + 1 < w.bounces;
+        if (ahead) {
+          CUDA_TRY(cudaEventRecord(b->shade_ev, st));
+          CUDA_TRY(cudaStreamWaitEvent(b->side, b->shade_ev, 0));
+          trace(k + 1, b->side);
+          CUDA_TRY(cudaEventRecord(b->extend_ev, b->side));
+        }
         if (S > 0) {
           LaunchOcclude(b->dev, pb, wc, k, S, static_cast<int>(std::min<int64_t>(int64_t(w.paths) * S, INT32_MAX)),
                         isect, stats_on, tree_nodes, st);
@@ -376,8 +400,9 @@ void RenderBatch(MuonBatch *b, const MuonRenderParams *params, double *const *d_
         }
         LaunchFold(pb, wc, k, S, w.paths, st);
         ++launches;
+        if (ahead) CUDA_TRY(cudaStreamWaitEvent(st, b->extend_ev, 0));
       }
-      LaunchFilmBatch(d_scenes, wsegs, w.nseg, w.pixels, pb, st);
+      LaunchFilmBatch(d_scenes, wsegs, w.nseg, w.pixels, pbs[0], st);
       ++launches;
       CUDA_TRY(cudaEventRecordWithFlags(b->wave_done[wi], st, cudaEventRecordExternal));
     }
