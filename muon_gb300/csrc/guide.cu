@@ -25,7 +25,16 @@ namespace {
 using namespace guide;
 
 constexpr int kThreads = 256;
-constexpr int kChunk = 512;  // samples per weight-gradient partial
+// Weight gradients are partial sums of at most kMaxChunks chunks of samples
+// (two blocks for each of 152 SMs), reduced in order afterwards. Fixed chunks
+// of 512 samples left a batch of 65,536 with 128 blocks: a 64 x 64 layer 57 us,
+// now 24, the first 123, now 86.
+constexpr int kMaxChunks = 304;
+inline int ChunkSamples(int batch) {
+  const int c = (batch + kMaxChunks - 1) / kMaxChunks;
+  return (std::max(c, 64) + 31) / 32 * 32;
+}
+inline int Chunks(int batch) { return (batch + ChunkSamples(batch) - 1) / ChunkSamples(batch); }
 
 // ---- packing and initialisation ------------------------------------------------
 // The inference image (guide_mlp.cuh): one thread per 16-byte chunk of a
@@ -140,56 +149,96 @@ __global__ void SampleKernel(const float *mix, int n, const float *u, float *dir
   pdf[i] = MixturePdf(mx, wx, wy, wz);
 }
 
-// ---- training: forward ----------------------------------------------------------
-// y[b][n] = act(sum_k x[b][k] w[k][n] + bias[n]) for a tile of 64 samples;
-// with kBlob, x is the one-blob encoding of features (batch x 8).
-template <bool kBlob, bool kRelu>
-__global__ void __launch_bounds__(kThreads) FwdLayerKernel(const float *x, const float *w, const float *bias, int K,
-                                                           int N, float *y, int batch) {
-  __shared__ float xs[64][33];
-  __shared__ __align__(16) float ws[32][64];
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int b0 = blockIdx.x * 64;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 32) {
-    for (int i = tid; i < 64 * 32; i += kThreads) {
-      const int r = i >> 5, c = i & 31, b = b0 + r, k = k0 + c;
-      float v = 0.0f;
-      if (b < batch) {
-        if (kBlob) v = Blob(x[static_cast<int64_t>(b) * kFeatures + k / kBins], k % kBins);
-        else v = x[static_cast<int64_t>(b) * K + k];
-      }
-      xs[r][c] = v;
-    }
-    for (int i = tid; i < 32 * 64; i += kThreads) {
-      const int r = i >> 6, c = i & 63;
-      ws[r][c] = c < N ? w[(k0 + r) * N + c] : 0.0f;
-    }
-    __syncthreads();
+// ---- training: layer products -----------------------------------------------------
+// The forward and the data-gradient kernels multiply a tile of 128 samples by a
+// 64 x 64 weight block with 128 threads, 8 x 8 outputs each, 32 inputs at a
+// time. Both operands lie in shared memory with the summed index outermost, so
+// that a thread's 16 operands of one step are four 16-byte loads for 64
+// multiply-adds (4 x 4 outputs took five loads for 16). The 128-sample rows are
+// stored with bits 2..4 of the column flipped by bits 2..4 of the row: writes
+// of a transposed tile then hit all banks, and groups of four stay together.
+// Every output sums its inputs in order, as one chain of multiply-adds. Bound
+// by the FP32 units and, at 512 tiles, by the wait for each piece: 65,536
+// samples x 64 x 64 forward 27 -> 20 us, backward 38 -> 22 (0.54 GFLOP, 27
+// TFLOP/s).
+constexpr int kTile = 128, kTileThreads = 128, kStep = 32;
+
+__device__ __forceinline__ int Swizzle(int row) { return ((row >> 2) & 7) << 2; }
+
+// acc[i][j] += sum over kStep rows r of xs[r][8 ty + i] * ws[r][8 tx + j].
+__device__ __forceinline__ void TileProduct(const float (*xs)[kTile], const float (*ws)[64], int ty, int tx,
+                                            bool ws_swizzled, float (&acc)[8][8]) {
 #pragma unroll 8
-    for (int kk = 0; kk < 32; ++kk) {
-      float a[4], bb[4];
+  for (int r = 0; r < kStep; ++r) {
+    const int sw = Swizzle(r);
+    const float4 a0 = *reinterpret_cast<const float4 *>(&xs[r][(8 * ty) ^ sw]);
+    const float4 a1 = *reinterpret_cast<const float4 *>(&xs[r][(8 * ty + 4) ^ sw]);
+    const int wsw = ws_swizzled ? sw : 0;
+    const float4 b0 = *reinterpret_cast<const float4 *>(&ws[r][(8 * tx) ^ wsw]);
+    const float4 b1 = *reinterpret_cast<const float4 *>(&ws[r][(8 * tx + 4) ^ wsw]);
+    const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = xs[ty * 4 + i][kk];
-      LoadRow<4>(&ws[kk][tx * 4], bb);
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+  }
+}
+
+// xs[k][b] = x[b0 + b][k0 + k] for a 128 x 32 piece of a batch x 64 array.
+__device__ __forceinline__ void LoadTransposed(const float *x, int b0, int k0, int batch, float (*xs)[kTile]) {
+  const int c4 = threadIdx.x & 7, r0 = threadIdx.x >> 3;  // 8 vectors a row, 16 rows at a time
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * bb[j];
+  for (int m = 0; m < kTile / 16; ++m) {
+    const int row = r0 + 16 * m, b = b0 + row;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (b < batch) v = *reinterpret_cast<const float4 *>(x + static_cast<int64_t>(b) * kWidth + k0 + 4 * c4);
+    const int col = row ^ (c4 << 2);
+    xs[4 * c4][col] = v.x, xs[4 * c4 + 1][col] = v.y, xs[4 * c4 + 2][col] = v.z, xs[4 * c4 + 3][col] = v.w;
+  }
+}
+
+// ---- training: forward ----------------------------------------------------------
+// y[b][n] = act(sum_k x[b][k] w[k][n] + bias[n]), 64 outputs; with kBlob, x is
+// the one-blob encoding of features (batch x 8), one feature per step.
+template <bool kBlob, bool kRelu>
+__global__ void __launch_bounds__(kTileThreads) FwdLayerKernel(const float *x, const float *w, const float *bias, int K,
+                                                               float *y, int batch) {
+  static_assert(kBins == kStep && kWidth == 64 && kOut == 64, "one feature a step, 64 outputs");
+  __shared__ __align__(16) float xs[kStep][kTile];
+  __shared__ __align__(16) float ws[kStep][64];
+  const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
+  const int b0 = blockIdx.x * kTile;
+  float acc[8][8] = {};
+  for (int k0 = 0; k0 < K; k0 += kStep) {
+    if (kBlob) {
+      const int b = b0 + tid;
+      const bool on = b < batch;
+      const float f = on ? x[static_cast<int64_t>(b) * kFeatures + k0 / kBins] : 0.0f;
+#pragma unroll 8
+      for (int k = 0; k < kBins; ++k) xs[k][tid ^ Swizzle(k)] = on ? Blob(f, k) : 0.0f;
+    } else {
+      LoadTransposed(x, b0, k0, batch, xs);
     }
+#pragma unroll
+    for (int i = tid; i < kStep * 16; i += kTileThreads)
+      reinterpret_cast<float4 *>(&ws[0][0])[i] = reinterpret_cast<const float4 *>(w + k0 * 64)[i];
+    __syncthreads();
+    TileProduct(xs, ws, ty, tx, false, acc);
     __syncthreads();
   }
+  float bb[8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int b = b0 + ty * 4 + i;
+  for (int j = 0; j < 8; ++j) bb[j] = bias[8 * tx + j];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int b = b0 + 8 * ty + i;
     if (b >= batch) continue;
+    float v[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = tx * 4 + j;
-      if (c >= N) continue;
-      float v = acc[i][j] + bias[c];
-      y[static_cast<int64_t>(b) * N + c] = kRelu ? fmaxf(v, 0.0f) : v;
-    }
+    for (int j = 0; j < 8; ++j) v[j] = kRelu ? fmaxf(acc[i][j] + bb[j], 0.0f) : acc[i][j] + bb[j];
+    float4 *o = reinterpret_cast<float4 *>(y + static_cast<int64_t>(b) * 64 + 8 * tx);
+    o[0] = make_float4(v[0], v[1], v[2], v[3]), o[1] = make_float4(v[4], v[5], v[6], v[7]);
   }
 }
 
@@ -201,154 +250,212 @@ __global__ void __launch_bounds__(kThreads) FwdLayerKernel(const float *x, const
 // gradient of log p_i follows oracle/guiding.py (loss_grad), through
 // s = exp(b) (inside the clip range), the tangent projection pu = u - (u.mu) mu
 // and mu = m / |m|.
+// Eight lanes per sample, one per lobe: a lane reads and writes its lobe's 32
+// bytes (a thread per sample read rows 256 bytes apart and walked the lobes in
+// turn: 50 us for 65,536 samples, now 19).
+__device__ __forceinline__ float LobeSum(float v) {
+  for (int o = 1; o < kLobes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ float LobeMax(float v) {
+  for (int o = 1; o < kLobes; o <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
 __global__ void __launch_bounds__(kThreads) LossKernel(float *z, const float *dirs, const float *weights, int batch,
                                                        double *loss_out) {
-  __shared__ double red[kThreads];
-  const int b = blockIdx.x * kThreads + threadIdx.x;
-  double loss = 0.0;
-  if (b < batch) {
-    float *r = z + static_cast<int64_t>(b) * kOut;
-    const float w[3] = {dirs[3 * b], dirs[3 * b + 1], dirs[3 * b + 2]};
-    const float wt = weights[b];
-    float amax = -INFINITY;
-    for (int i = 0; i < kLobes; ++i) amax = fmaxf(amax, r[kLobeOut * i]);
-    float se = 0.0f;
-    for (int i = 0; i < kLobes; ++i) se += expf(r[kLobeOut * i] - amax);
-    const float lse = amax + logf(se);
-    // pass 1: log of each lobe's share of q (-inf where the lobe is zero)
-    float t[kLobes];
-    const float log_keep = logf(1.0f - kEpsUniform), t_uniform = logf(kEpsUniform * 0.25f / kPi);
-    float tmax = t_uniform;
-    for (int i = 0; i < kLobes; ++i) {
-      const float *ri = r + kLobeOut * i;
-      t[i] = -INFINITY;
-      const float n2 = ri[1] * ri[1] + ri[2] * ri[2] + ri[3] * ri[3];
-      float mu[3] = {0.0f, 0.0f, 1.0f};
-      if (n2 > 1e-24f) {
-        const float k = 1.0f / sqrtf(n2);
-        mu[0] = ri[1] * k, mu[1] = ri[2] * k, mu[2] = ri[3] * k;
-      }
-      const float c = mu[0] * w[0] + mu[1] * w[1] + mu[2] * w[2];
-      if (!(c > kCMin)) continue;
-      const float s = expf(fminf(fmaxf(ri[4], kBMin), kBMax));
-      const float um = ri[5] * mu[0] + ri[6] * mu[1] + ri[7] * mu[2];
-      float pu[3], v[3], p2 = 0.0f, v2 = 0.0f, d = 0.0f;
-      for (int k = 0; k < 3; ++k) {
-        pu[k] = ri[5 + k] - um * mu[k];
-        v[k] = w[k] / c - mu[k];
-        p2 += pu[k] * pu[k], v2 += v[k] * v[k], d += pu[k] * v[k];
-      }
-      const float logp = 0.5f * logf(s) + 0.5f * logf(s + p2) - logf(2.0f * kPi) - 0.5f * (s * v2 + d * d) -
-                         3.0f * logf(c);
-      t[i] = log_keep + (ri[0] - lse) + logp;
-      tmax = fmaxf(tmax, t[i]);
+  static_assert(kThreads == kLobes * kGuideLossSamples, "one loss sum per block");
+  __shared__ double red[kGuideLossSamples];
+  const int lobe = threadIdx.x & (kLobes - 1), sample = threadIdx.x / kLobes;
+  const int b = blockIdx.x * kGuideLossSamples + sample;
+  const bool on = b < batch;
+  float r[kLobeOut] = {};
+  float w[3] = {0.0f, 0.0f, 1.0f}, wt = 0.0f;
+  float4 *row = reinterpret_cast<float4 *>(z + static_cast<int64_t>(b) * kOut + kLobeOut * lobe);
+  if (on) {
+    const float4 r0 = row[0], r1 = row[1];
+    r[0] = r0.x, r[1] = r0.y, r[2] = r0.z, r[3] = r0.w, r[4] = r1.x, r[5] = r1.y, r[6] = r1.z, r[7] = r1.w;
+    w[0] = dirs[3 * static_cast<int64_t>(b)], w[1] = dirs[3 * static_cast<int64_t>(b) + 1];
+    w[2] = dirs[3 * static_cast<int64_t>(b) + 2];
+    wt = weights[b];
+  }
+  const float amax = LobeMax(r[0]);
+  const float lse = amax + logf(LobeSum(expf(r[0] - amax)));
+  // log of the lobe's share of q (-inf where the lobe is zero)
+  const float log_keep = logf(1.0f - kEpsUniform), t_uniform = logf(kEpsUniform * 0.25f / kPi);
+  float t = -INFINITY;
+  const float n2 = r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+  const float nrm = sqrtf(n2);
+  float mu[3] = {0.0f, 0.0f, 1.0f};
+  if (n2 > 1e-24f) mu[0] = r[1] / nrm, mu[1] = r[2] / nrm, mu[2] = r[3] / nrm;
+  const float c = mu[0] * w[0] + mu[1] * w[1] + mu[2] * w[2];
+  const float s = expf(fminf(fmaxf(r[4], kBMin), kBMax));
+  const float um = r[5] * mu[0] + r[6] * mu[1] + r[7] * mu[2];
+  float pu[3], v[3], p2 = 0.0f, v2 = 0.0f, d = 0.0f, vw = 0.0f, pw = 0.0f;
+  if (c > kCMin) {
+    for (int k = 0; k < 3; ++k) {
+      pu[k] = r[5 + k] - um * mu[k];
+      v[k] = w[k] / c - mu[k];
+      p2 += pu[k] * pu[k], v2 += v[k] * v[k], d += pu[k] * v[k];
+      vw += v[k] * w[k], pw += pu[k] * w[k];
     }
-    float qs = expf(t_uniform - tmax);
-    for (int i = 0; i < kLobes; ++i) qs += expf(t[i] - tmax);
-    const float logq = tmax + logf(qs);
-    loss = -static_cast<double>(wt) * logq;
+    const float logp = 0.5f * logf(s) + 0.5f * logf(s + p2) - logf(2.0f * kPi) - 0.5f * (s * v2 + d * d) - 3.0f * logf(c);
+    t = log_keep + (r[0] - lse) + logp;
+  }
+  const float tmax = fmaxf(t_uniform, LobeMax(t));
+  const float logq = tmax + logf(expf(t_uniform - tmax) + LobeSum(expf(t - tmax)));
+  const float resp = expf(t - logq);
+  const float rsum = LobeSum(resp);
+  if (on) {
     const float coef = -wt / static_cast<float>(batch);
-    float resp[kLobes], rsum = 0.0f;
-    for (int i = 0; i < kLobes; ++i) {
-      resp[i] = expf(t[i] - logq);
-      rsum += resp[i];
-    }
-    // pass 2: gradients, written over the raw outputs
-    for (int i = 0; i < kLobes; ++i) {
-      float *ri = r + kLobeOut * i;
-      const float pi = expf(ri[0] - lse);
-      float g[kLobeOut] = {coef * (resp[i] - pi * rsum), 0, 0, 0, 0, 0, 0, 0};
-      const float n2 = ri[1] * ri[1] + ri[2] * ri[2] + ri[3] * ri[3];
-      float mu[3] = {0.0f, 0.0f, 1.0f};
-      const float nrm = sqrtf(n2);
-      if (n2 > 1e-24f) mu[0] = ri[1] / nrm, mu[1] = ri[2] / nrm, mu[2] = ri[3] / nrm;
-      const float c = mu[0] * w[0] + mu[1] * w[1] + mu[2] * w[2];
-      if (resp[i] > 0.0f && c > kCMin) {
-        const float cr = coef * resp[i];
-        const float braw = ri[4];
-        const float s = expf(fminf(fmaxf(braw, kBMin), kBMax));
-        const float um = ri[5] * mu[0] + ri[6] * mu[1] + ri[7] * mu[2];
-        float pu[3], v[3], p2 = 0.0f, v2 = 0.0f, d = 0.0f, vw = 0.0f, pw = 0.0f;
+    const float pi = expf(r[0] - lse);
+    float g[kLobeOut] = {coef * (resp - pi * rsum), 0, 0, 0, 0, 0, 0, 0};
+    if (resp > 0.0f && c > kCMin) {
+      const float cr = coef * resp;
+      const float sp2 = s + p2;
+      if (r[4] > kBMin && r[4] < kBMax) g[4] = cr * (0.5f + 0.5f * s / sp2 - 0.5f * s * v2);
+      for (int k = 0; k < 3; ++k) g[5 + k] = cr * (pu[k] / sp2 - d * v[k]);
+      if (n2 > 1e-24f) {
+        const float ic2 = 1.0f / (c * c);
+        float gm[3], dot = 0.0f;
         for (int k = 0; k < 3; ++k) {
-          pu[k] = ri[5 + k] - um * mu[k];
-          v[k] = w[k] / c - mu[k];
-          p2 += pu[k] * pu[k], v2 += v[k] * v[k], d += pu[k] * v[k];
-          vw += v[k] * w[k], pw += pu[k] * w[k];
+          gm[k] = -um * pu[k] / sp2 + s * (vw * w[k] * ic2 + v[k]) + d * (um * v[k] + pw * w[k] * ic2 + pu[k]) -
+                  3.0f * w[k] / c;
+          dot += gm[k] * mu[k];
         }
-        const float sp2 = s + p2;
-        if (braw > kBMin && braw < kBMax) g[4] = cr * (0.5f + 0.5f * s / sp2 - 0.5f * s * v2);
-        for (int k = 0; k < 3; ++k) g[5 + k] = cr * (pu[k] / sp2 - d * v[k]);
-        if (n2 > 1e-24f) {
-          const float ic2 = 1.0f / (c * c);
-          float gm[3], dot = 0.0f;
-          for (int k = 0; k < 3; ++k) {
-            gm[k] = -um * pu[k] / sp2 + s * (vw * w[k] * ic2 + v[k]) + d * (um * v[k] + pw * w[k] * ic2 + pu[k]) -
-                    3.0f * w[k] / c;
-            dot += gm[k] * mu[k];
-          }
-          for (int k = 0; k < 3; ++k) g[1 + k] = cr * (gm[k] - dot * mu[k]) / nrm;
-        }
+        for (int k = 0; k < 3; ++k) g[1 + k] = cr * (gm[k] - dot * mu[k]) / nrm;
       }
-      for (int k = 0; k < kLobeOut; ++k) ri[k] = g[k];
     }
+    row[0] = make_float4(g[0], g[1], g[2], g[3]);
+    row[1] = make_float4(g[4], g[5], g[6], g[7]);
   }
-  red[threadIdx.x] = loss;
+  if (lobe == 0) red[sample] = on ? -static_cast<double>(wt) * logq : 0.0;
   __syncthreads();
-  for (int o = kThreads / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    double sum = 0.0;
+    for (int i = 0; i < kGuideLossSamples; ++i) sum += red[i];
+    loss_out[blockIdx.x] = sum;
   }
-  if (threadIdx.x == 0) loss_out[blockIdx.x] = red[0];
 }
 
 // ---- training: backward -------------------------------------------------------------
-// dx[b][k] = (sum_n dz[b][n] w[k][n]) * (h[b][k] > 0), K = 64, N <= 64.
-__global__ void __launch_bounds__(kThreads) BwdDataKernel(const float *dz, const float *w, const float *h, int N,
-                                                          float *dx, int batch) {
-  __shared__ float ds[64][65];
-  __shared__ __align__(16) float wt[64][68];  // wt[n][k] = w[k][n], rows 16-byte aligned
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int b0 = blockIdx.x * 64;
-  for (int i = tid; i < 64 * 64; i += kThreads) {
-    const int r = i >> 6, c = i & 63, b = b0 + r;
-    ds[r][c] = (b < batch && c < N) ? dz[static_cast<int64_t>(b) * N + c] : 0.0f;
-    wt[c][r] = c < N ? w[r * N + c] : 0.0f;  // w row k = r, column n = c
-  }
-  __syncthreads();
-  float acc[4][4] = {};
-  for (int n = 0; n < N; ++n) {
-    float a[4], bb[4];
+// dx[b][k] = (sum_n dz[b][n] w[k][n]) * (h[b][k] > 0), 64 inputs and outputs.
+__global__ void __launch_bounds__(kTileThreads) BwdDataKernel(const float *dz, const float *w, const float *h,
+                                                              float *dx, int batch) {
+  __shared__ __align__(16) float ds[kStep][kTile];
+  __shared__ __align__(16) float wt[kStep][64];  // wt[n][k] = w[k][n], columns flipped as in ds
+  const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
+  const int b0 = blockIdx.x * kTile;
+  float acc[8][8] = {};
+  for (int n0 = 0; n0 < 64; n0 += kStep) {
+    LoadTransposed(dz, b0, n0, batch, ds);
+    const int c4 = tid & 7;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = ds[ty * 4 + i][n];
-    LoadRow<4>(&wt[n][tx * 4], bb);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * bb[j];
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int b = b0 + ty * 4 + i;
-    if (b >= batch) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int k = tx * 4 + j;
-      const int64_t o = static_cast<int64_t>(b) * kWidth + k;
-      dx[o] = h[o] > 0.0f ? acc[i][j] : 0.0f;
+    for (int m = 0; m < 4; ++m) {
+      const int k = (tid >> 3) + 16 * m;
+      const float4 v = *reinterpret_cast<const float4 *>(w + k * 64 + n0 + 4 * c4);
+      const int col = k ^ (c4 << 2);
+      wt[4 * c4][col] = v.x, wt[4 * c4 + 1][col] = v.y, wt[4 * c4 + 2][col] = v.z, wt[4 * c4 + 3][col] = v.w;
     }
+    __syncthreads();
+    TileProduct(ds, wt, ty, tx, true, acc);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int b = b0 + 8 * ty + i;
+    if (b >= batch) continue;
+    const int64_t o = static_cast<int64_t>(b) * kWidth + 8 * tx;
+    const float4 h0 = *reinterpret_cast<const float4 *>(h + o), h1 = *reinterpret_cast<const float4 *>(h + o + 4);
+    *reinterpret_cast<float4 *>(dx + o) = make_float4(h0.x > 0.0f ? acc[i][0] : 0.0f, h0.y > 0.0f ? acc[i][1] : 0.0f,
+                                                      h0.z > 0.0f ? acc[i][2] : 0.0f, h0.w > 0.0f ? acc[i][3] : 0.0f);
+    *reinterpret_cast<float4 *>(dx + o + 4) =
+        make_float4(h1.x > 0.0f ? acc[i][4] : 0.0f, h1.y > 0.0f ? acc[i][5] : 0.0f, h1.z > 0.0f ? acc[i][6] : 0.0f,
+                    h1.w > 0.0f ? acc[i][7] : 0.0f);
   }
 }
 
-// Per chunk of samples: partial[k * N + n] = sum_b x[b][k] dz[b][n] and the
-// bias part partial[K * N + n] = sum_b dz[b][n]. Each thread owns a TK x TN
-// block of outputs.
-// Weight and bias gradients of one layer over one chunk of kChunk samples:
-// partial[chunk][k][n] = sum over the chunk's samples of x[b][k] dz[b][n].
+// Weight and bias gradients of a 64 x 64 layer over one chunk of samples:
+// partial[k][n] = sum_b x[b][k] dz[b][n], then sum_b dz[b][n]. Four groups of 64
+// threads take every fourth sample of the staged 32, 8 x 8 gradients a thread
+// (four 16-byte loads for 64 multiply-adds), and their sums are added in order
+// at the end; the next 32 samples load meanwhile.
+constexpr int kSlices = kThreads / 64;
+__global__ void __launch_bounds__(kThreads, 2) WgradSquareKernel(const float *x, const float *dz, int batch,
+                                                                 int chunk, float *partial, int layer_off) {
+  constexpr int kRows = 32, kVec = kRows * 64 / 4 / kThreads;  // rows staged, vectors a thread
+  __shared__ __align__(16) float xs[kRows][64], ds[kRows][64];
+  __shared__ float sums[64][65];
+  const int tid = threadIdx.x, slice = tid >> 6, kg = (tid >> 3) & 7, ng = tid & 7;
+  const int b0 = blockIdx.x * chunk, b1 = min(batch, b0 + chunk);
+  float acc[8][8] = {}, bacc[8] = {};
+  float4 px[kVec], pd[kVec];
+  auto fetch = [&](int s0) {
+#pragma unroll
+    for (int m = 0; m < kVec; ++m) {
+      const int i = tid + m * kThreads, b = s0 + (i >> 4);
+      px[m] = pd[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (b < b1) {
+        px[m] = reinterpret_cast<const float4 *>(x + static_cast<int64_t>(b) * 64)[i & 15];
+        pd[m] = reinterpret_cast<const float4 *>(dz + static_cast<int64_t>(b) * 64)[i & 15];
+      }
+    }
+  };
+  fetch(b0);
+  for (int s0 = b0; s0 < b1; s0 += kRows) {
+#pragma unroll
+    for (int m = 0; m < kVec; ++m) {
+      const int i = tid + m * kThreads;
+      reinterpret_cast<float4 *>(&xs[0][0])[i] = px[m];
+      reinterpret_cast<float4 *>(&ds[0][0])[i] = pd[m];
+    }
+    __syncthreads();
+    if (s0 + kRows < b1) fetch(s0 + kRows);
+#pragma unroll 4
+    for (int r = slice; r < kRows; r += kSlices) {
+      float a[8], d[8];
+      LoadRow<8>(&xs[r][8 * kg], a);
+      LoadRow<8>(&ds[r][8 * ng], d);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], d[j], acc[i][j]);
+      if (kg == 0)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) bacc[j] += d[j];
+    }
+    __syncthreads();
+  }
+  // rows 0..63: weights; the bias row through the last column
+  float *p = partial + static_cast<int64_t>(blockIdx.x) * kParams + layer_off;
+  for (int q = 0; q < kSlices; ++q) {
+    if (slice == q) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float &o = sums[8 * kg + i][8 * ng + j];
+          o = q == 0 ? acc[i][j] : o + acc[i][j];
+        }
+      if (kg == 0)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float &o = sums[8 * ng + j][64];
+          o = q == 0 ? bacc[j] : o + bacc[j];
+        }
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < 64 * 64; i += kThreads) p[i] = sums[i >> 6][i & 63];
+  if (tid < 64) p[64 * 64 + tid] = sums[tid][64];
+}
+
+// The same for the first layer, whose inputs are the one-blob encoding.
 // Each thread owns a TK x TN tile of the K x N gradient; 32 samples at a time
 // are staged in shared memory (rows of K and N floats, read back as vectors).
 template <bool kBlob, int K, int N, int TK, int TN>
-__global__ void __launch_bounds__(kThreads) WgradKernel(const float *x, const float *dz, int batch, float *partial,
-                                                        int stride, int layer_off) {
+__global__ void __launch_bounds__(kThreads) WgradKernel(const float *x, const float *dz, int batch, int chunk,
+                                                        float *partial, int stride, int layer_off) {
   static_assert((K / TK) * (N / TN) == kThreads, "thread tiling");
   static_assert(K % 4 == 0 && N % 4 == 0, "rows of whole 16-byte vectors");
   __shared__ __align__(16) float xs[32][K];
@@ -356,10 +463,10 @@ __global__ void __launch_bounds__(kThreads) WgradKernel(const float *x, const fl
   __shared__ float fs[32][kFeatures];  // one-blob input: the slab's features
   const int tid = threadIdx.x;
   const int kg = tid / (N / TN), ng = tid % (N / TN);
-  const int b0 = blockIdx.x * kChunk;
+  const int b0 = blockIdx.x * chunk;
   float acc[TK][TN] = {};
   float bacc = 0.0f;
-  for (int s0 = b0; s0 < b0 + kChunk && s0 < batch; s0 += 32) {
+  for (int s0 = b0; s0 < b0 + chunk && s0 < batch; s0 += 32) {
     if (kBlob) {
       for (int i = tid; i < 32 * kFeatures; i += kThreads) {
         const int r = i / kFeatures, b = s0 + r;
@@ -502,10 +609,10 @@ void LaunchGuideSample(const float *raw, int n, const float *u, float *mix, floa
 }
 
 size_t GuideTrainBytes(int batch) {
-  const size_t chunks = (batch + kChunk - 1) / kChunk;
+  const size_t chunks = static_cast<size_t>(Chunks(batch));
   return sizeof(float) * (4ull * batch * kWidth + static_cast<size_t>(batch) * kOut + 2ull * batch * kWidth +
                           chunks * kParams + kParams) +
-         sizeof(double) * (batch / kThreads + 2 + kSumBlocks) + 256 * 9;
+         sizeof(double) * (batch / kGuideLossSamples + 2 + kSumBlocks) + 256 * 10;
 }
 
 void GuideTrainCarve(void *base, int batch, GuideTrainBuffers *out) {
@@ -520,39 +627,37 @@ void GuideTrainCarve(void *base, int batch, GuideTrainBuffers *out) {
   out->z = reinterpret_cast<float *>(take(sizeof(float) * batch * kOut));
   out->dz[0] = reinterpret_cast<float *>(take(sizeof(float) * batch * kWidth));
   out->dz[1] = reinterpret_cast<float *>(take(sizeof(float) * batch * kWidth));
-  out->chunks = (batch + kChunk - 1) / kChunk;
+  out->chunks = Chunks(batch);
   out->partial = reinterpret_cast<float *>(take(sizeof(float) * out->chunks * kParams));
   out->grad = reinterpret_cast<float *>(take(sizeof(float) * kParams));
-  out->loss = reinterpret_cast<double *>(take(sizeof(double) * (batch / kThreads + 2)));
+  out->loss = reinterpret_cast<double *>(take(sizeof(double) * (batch / kGuideLossSamples + 2)));
   out->wsum = reinterpret_cast<double *>(take(sizeof(double) * kSumBlocks));
 }
 
 void LaunchGuideGradients(const float *params, const float *features, const float *dirs, const float *weights,
                           int batch, const GuideTrainBuffers &tb, cudaStream_t st) {
-  const unsigned tiles = Grid(batch, 64);
+  const unsigned tiles = Grid(batch, kTile);
   auto W = [&](int l) { return params + MasterOffset(l); };
   auto B = [&](int l) { return params + MasterOffset(l) + In(l) * Out(l); };
-  FwdLayerKernel<true, true><<<tiles, kThreads, 0, st>>>(features, W(0), B(0), kIn, kWidth, tb.h[1], batch);
+  FwdLayerKernel<true, true><<<tiles, kTileThreads, 0, st>>>(features, W(0), B(0), kIn, tb.h[1], batch);
   for (int l = 1; l < 4; ++l)
-    FwdLayerKernel<false, true><<<tiles, kThreads, 0, st>>>(tb.h[l], W(l), B(l), kWidth, kWidth, tb.h[l + 1], batch);
-  FwdLayerKernel<false, false><<<tiles, kThreads, 0, st>>>(tb.h[4], W(4), B(4), kWidth, kOut, tb.z, batch);
-  LossKernel<<<Grid(batch, kThreads), kThreads, 0, st>>>(tb.z, dirs, weights, batch, tb.loss);
+    FwdLayerKernel<false, true><<<tiles, kTileThreads, 0, st>>>(tb.h[l], W(l), B(l), kWidth, tb.h[l + 1], batch);
+  FwdLayerKernel<false, false><<<tiles, kTileThreads, 0, st>>>(tb.h[4], W(4), B(4), kWidth, tb.z, batch);
+  LossKernel<<<Grid(batch, kGuideLossSamples), kThreads, 0, st>>>(tb.z, dirs, weights, batch, tb.loss);
   const unsigned chunks = static_cast<unsigned>(tb.chunks);
-  // layer 4: 64 x 64
-  WgradKernel<false, kWidth, kOut, 4, 4><<<chunks, kThreads, 0, st>>>(tb.h[4], tb.z, batch, tb.partial, kParams,
-                                                                       MasterOffset(4));
-  BwdDataKernel<<<tiles, kThreads, 0, st>>>(tb.z, W(4), tb.h[4], kOut, tb.dz[0], batch);
-  // layers 3..1: 64 x 64
+  const int chunk = ChunkSamples(batch);
+  // layers 4..1: 64 x 64
+  const float *dz = tb.z;
   int cur = 0;
-  for (int l = 3; l >= 1; --l) {
-    WgradKernel<false, kWidth, kWidth, 4, 4><<<chunks, kThreads, 0, st>>>(tb.h[l], tb.dz[cur], batch, tb.partial,
-                                                                         kParams, MasterOffset(l));
-    BwdDataKernel<<<tiles, kThreads, 0, st>>>(tb.dz[cur], W(l), tb.h[l], kWidth, tb.dz[cur ^ 1], batch);
+  for (int l = 4; l >= 1; --l) {
+    WgradSquareKernel<<<chunks, kThreads, 0, st>>>(tb.h[l], dz, batch, chunk, tb.partial, MasterOffset(l));
+    BwdDataKernel<<<tiles, kTileThreads, 0, st>>>(dz, W(l), tb.h[l], tb.dz[cur], batch);
+    dz = tb.dz[cur];
     cur ^= 1;
   }
   // layer 0: one-blob input, 256 x 64
-  WgradKernel<true, kIn, kWidth, 8, 8><<<chunks, kThreads, 0, st>>>(features, tb.dz[cur], batch, tb.partial,
-                                                                    kParams, MasterOffset(0));
+  WgradKernel<true, kIn, kWidth, 8, 8><<<chunks, kThreads, 0, st>>>(features, dz, batch, chunk, tb.partial, kParams,
+                                                                    MasterOffset(0));
   ReduceKernel<<<Grid(kParams, 256), 256, 0, st>>>(tb.partial, tb.chunks, tb.grad);
 }
 

@@ -92,6 +92,9 @@ void LaunchGuideForward(const void *img, const float *features, int n, float *ou
 void LaunchGuideSample(const float *raw, int n, const float *u, float *mix, float *dirs, float *pdf,
                        cudaStream_t st);
 
+// Consecutive samples whose losses the training step adds up (GuideTrainBuffers::loss).
+constexpr int kGuideLossSamples = 32;
+
 // Working memory of one training step over `batch` samples.
 struct GuideTrainBuffers {
   float *h[5];      // inputs of layers 1..4 (h[0] unused: the one-blob input is recomputed), batch x 64
@@ -99,7 +102,7 @@ struct GuideTrainBuffers {
   float *dz[2];     // batch x 64 gradients (ping-pong)
   float *partial;   // per chunk: all weight and bias gradients
   float *grad;      // guide::kParams
-  double *loss;     // loss sum of every 256 consecutive samples
+  double *loss;     // loss sum of every kGuideLossSamples consecutive samples
   double *wsum;     // partial sums of the training weights (LaunchGuideGather)
   int32_t chunks;
 };

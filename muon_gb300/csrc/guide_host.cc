@@ -198,8 +198,8 @@ int muon_gpu_guide_train(MuonGuide *guide, int32_t steps, double *loss) {
     LaunchGuidePack(guide->params.as<float>(), guide->wt.ptr, st);
     CUDA_TRY(cudaGetLastError());
     if (loss) {
-      std::vector<double> parts(batch / 256 + 1, 0.0);
-      const size_t nparts = (batch + 255) / 256;
+      const size_t nparts = (static_cast<size_t>(batch) + kGuideLossSamples - 1) / kGuideLossSamples;
+      std::vector<double> parts(nparts, 0.0);
       CUDA_TRY(cudaMemcpyAsync(parts.data(), tb.loss, nparts * sizeof(double), cudaMemcpyDeviceToHost, st));
       CUDA_TRY(cudaStreamSynchronize(st));
       double sum = 0.0;
@@ -273,8 +273,8 @@ int muon_gpu_guide_gradients(MuonGuide *guide, const float *features, const floa
   try {
     CUDA_TRY(cudaSetDevice(guide->view.device));
     cudaStream_t st = guide->view.stream;
-    DeviceBuffer work;
-    work.Ensure(GuideTrainBytes(n));
+    DeviceBuffer work;  // from the device block cache, and back to it
+    EnsurePooled(work, GuideTrainBytes(n), guide->view.device);
     GuideTrainBuffers tb;
     GuideTrainCarve(work.ptr, n, &tb);
     guide->io_in.Ensure(sizeof(float) * n * guide::kFeatures);
@@ -288,10 +288,11 @@ int muon_gpu_guide_gradients(MuonGuide *guide, const float *features, const floa
                          guide->io_w.as<float>(), n, tb, st);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(grad, tb.grad, sizeof(float) * guide::kParams, cudaMemcpyDeviceToHost, st));
-    const size_t nparts = (n + 255) / 256;
+    const size_t nparts = (static_cast<size_t>(n) + kGuideLossSamples - 1) / kGuideLossSamples;
     std::vector<double> parts(nparts);
     CUDA_TRY(cudaMemcpyAsync(parts.data(), tb.loss, nparts * sizeof(double), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
+    PoolGive(work, guide->view.device);
     if (loss) {
       double sum = 0.0;
       for (double v : parts) sum += v;
