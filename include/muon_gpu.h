@@ -312,6 +312,14 @@ int muon_gpu_intersect(MuonScene *scene, const MuonRay *rays, int64_t n, int32_t
                        MuonHit *hits);
 int muon_gpu_occluded(MuonScene *scene, const MuonRay *rays, const float *max_distance, int64_t n,
                       int32_t intersect_mode, uint8_t *occluded);
+/* The same with every field in an array of its own (origins, directions,
+ * position and normal: 3 floats per ray), for callers that hold them so: no
+ * interleaving on either side. */
+int muon_gpu_intersect_arrays(MuonScene *scene, const float *origins, const float *directions, int64_t n,
+                              int32_t intersect_mode, float *distance, int32_t *prim_id, float *position,
+                              float *normal);
+int muon_gpu_occluded_arrays(MuonScene *scene, const float *origins, const float *directions,
+                             const float *max_distance, int64_t n, int32_t intersect_mode, uint8_t *occluded);
 
 /* No counterpart in the reference. For callers that must not allocate device
  * memory while rendering — a host application whose own allocator reserves

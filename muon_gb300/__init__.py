@@ -146,6 +146,11 @@ class FilmResult:
         check(load().muon_film_write(C.byref(f), C.c_float(gamma), path.encode()))
 
 
+def _vectors(a, n: int) -> np.ndarray:
+    """n vectors as contiguous float32 (n, 3), broadcast like an assignment."""
+    return np.ascontiguousarray(np.broadcast_to(np.asarray(a), (n, 3)), dtype=np.float32)
+
+
 # Below this many primitives the host builds the SAH tree faster than the
 # device's launches and synchronisations (measured on a GB300: 36 primitives
 # 0.20 ms on the host vs 0.39 ms on the device; 516 primitives 1.04 vs 0.55 ms).
@@ -241,27 +246,24 @@ class Scene:
         index in scene-file order, -1 on a miss.
         """
         n = len(origins)
-        rays = np.zeros((n, 6), dtype=np.float32)
-        rays[:, :3] = origins
-        rays[:, 3:] = directions
-        hits = np.zeros((n, 8), dtype=np.float32)
-        check(load().muon_gpu_intersect(self._h, rays.ctypes.data_as(C.POINTER(native.Ray)), n, intersect_mode,
-                                        hits.ctypes.data_as(C.POINTER(native.Hit))))
-        return hits[:, 0].copy(), hits[:, 1].view(np.int32).copy(), hits[:, 2:5].copy(), hits[:, 5:8].copy()
+        o, d = _vectors(origins, n), _vectors(directions, n)
+        distance, prim_id = np.empty(n, dtype=np.float32), np.empty(n, dtype=np.int32)
+        position, normal = np.empty((n, 3), dtype=np.float32), np.empty((n, 3), dtype=np.float32)
+        check(load().muon_gpu_intersect_arrays(self._h, o.ctypes.data, d.ctypes.data, n, intersect_mode,
+                                               distance.ctypes.data, prim_id.ctypes.data, position.ctypes.data,
+                                               normal.ctypes.data))
+        return distance, prim_id, position, normal
 
     def occluded(self, origins: np.ndarray, directions: np.ndarray, max_distance: np.ndarray,
                  intersect_mode: int = native.ISECT_EXACT) -> np.ndarray:
         """Any hit closer than max_distance (Structure::HasIntersection)."""
         n = len(origins)
-        rays = np.zeros((n, 6), dtype=np.float32)
-        rays[:, :3] = origins
-        rays[:, 3:] = directions
+        o, d = _vectors(origins, n), _vectors(directions, n)
         md = np.ascontiguousarray(max_distance, dtype=np.float32)
-        out = np.zeros(n, dtype=np.uint8)
-        check(load().muon_gpu_occluded(self._h, rays.ctypes.data_as(C.POINTER(native.Ray)),
-                                       md.ctypes.data_as(C.POINTER(C.c_float)), n, intersect_mode,
-                                       out.ctypes.data_as(C.POINTER(C.c_uint8))))
-        return out.astype(bool)
+        out = np.empty(n, dtype=bool)
+        check(load().muon_gpu_occluded_arrays(self._h, o.ctypes.data, d.ctypes.data, md.ctypes.data, n, intersect_mode,
+                                              out.ctypes.data))
+        return out
 
     def probe_traversal(self, params: native.RenderParams, rays_per_queue: int = 4096) -> dict:
         """Traversal work of a render counted by the host walk of sampled

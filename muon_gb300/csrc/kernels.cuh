@@ -165,11 +165,24 @@ void LaunchFilmBatch(const BatchScene *scenes, const BatchSeg *segs, int nseg, i
 // Grid of the persistent traversal kernels for the launches that follow
 // (0 restores the default of filling every SM once).
 void SetTraversalBlocksOverride(int blocks);
-// Ray-level queries for the batched Intersect/HasIntersection seams.
-void LaunchIntersectRays(const DevScene &s, const float *rays, int64_t n, int isect, float *out_hit,
+// Ray-level queries for the batched Intersect/HasIntersection seams. Ray i's
+// origin and direction start at float `stride` * i of their arrays (6 for
+// MuonRay, 3 for arrays of their own), the fields of hit i at `stride` * i and
+// the vectors at `stride3` * i (8 and 8 for MuonHit, 1 and 3).
+struct QueryRays {
+  const float *origin, *direction;
+  int32_t stride;
+};
+struct QueryHits {
+  float *distance;
+  int32_t *prim_id;
+  float *position, *normal;
+  int32_t stride, stride3;
+};
+void LaunchIntersectRays(const DevScene &s, const QueryRays &q, int n, int isect, const QueryHits &out,
                          cudaStream_t st);
-void LaunchOccludedRays(const DevScene &s, const float *rays, const float *maxd, int64_t n, int isect,
-                        uint8_t *out, cudaStream_t st);
+void LaunchOccludedRays(const DevScene &s, const QueryRays &q, const float *maxd, int n, int isect, uint8_t *out,
+                        cudaStream_t st);
 
 // Measurement: a sample of bounce `bounce`'s closest-hit (kind 0) or shadow
 // (kind 1) queue, up to m rays, into out (1 + 2m float4s; see SampleQueueKernel).

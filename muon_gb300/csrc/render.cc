@@ -1199,11 +1199,68 @@ int muon_gpu_render(MuonScene *scene, const MuonRenderParams *params, MuonFilm *
   return MUON_OK;
 }
 
-int muon_gpu_intersect(MuonScene *scene, const MuonRay *rays, int64_t n, int32_t intersect_mode, MuonHit *hits) {
-  if (!scene || (n > 0 && (!rays || !hits)) || n < 0) return Fail(MUON_ERR_INVALID_ARG, "bad argument");
+namespace {
+
+// Rays of one launch of a query (its kernels count in 32 bits).
+constexpr int64_t kQueryLaunch = int64_t(1) << 28;
+
+// A query's checks; returns MUON_OK with nothing to do where n is 0.
+int CheckQuery(const MuonScene *scene, bool arrays, int64_t n, int32_t intersect_mode) {
+  if (!scene || (n > 0 && !arrays) || n < 0) return Fail(MUON_ERR_INVALID_ARG, "bad argument");
   if (intersect_mode < MUON_ISECT_FAST || intersect_mode > MUON_ISECT_EXACT)
     return Fail(MUON_ERR_INVALID_ARG, "unknown intersect_mode");
-  if (n == 0) return MUON_OK;
+  return MUON_OK;
+}
+
+// Closest hits of the n rays at `rays` (device) into `hits` (device).
+void IntersectOnDevice(MuonScene *scene, const QueryRays &rays, int64_t n, int32_t mode, const QueryHits &hits) {
+  for (int64_t i = 0; i < n; i += kQueryLaunch) {
+    const QueryRays q{rays.origin + rays.stride * i, rays.direction + rays.stride * i, rays.stride};
+    const QueryHits h{hits.distance + hits.stride * i, hits.prim_id + hits.stride * i, hits.position + hits.stride3 * i,
+                      hits.normal + hits.stride3 * i, hits.stride, hits.stride3};
+    LaunchIntersectRays(scene->dev, q, static_cast<int>(std::min(n - i, kQueryLaunch)), mode, h, scene->stream);
+  }
+  CUDA_TRY(cudaGetLastError());
+}
+
+// Few rays go through one staging block on the host: each copy to or from
+// pageable memory costs more than its bytes (1,000 rays: 119 us in one copy
+// each way, 129 in two and four).
+constexpr int64_t kQueryStaged = 8192;
+
+// Origins, directions and (optional) limits of n rays to the device, one array
+// after the other; through `stage` (room for all of them) if it is not null.
+void SendRays(MuonScene *scene, const float *origins, const float *directions, const float *limits, int64_t n,
+              float *stage) {
+  const size_t f = sizeof(float);
+  float *dst = scene->ray_in.as<float>();
+  if (stage) {
+    std::memcpy(stage, origins, 3 * n * f);
+    std::memcpy(stage + 3 * n, directions, 3 * n * f);
+    if (limits) std::memcpy(stage + 6 * n, limits, n * f);
+    CUDA_TRY(cudaMemcpyAsync(dst, stage, (limits ? 7 : 6) * n * f, cudaMemcpyHostToDevice, scene->stream));
+    return;
+  }
+  CUDA_TRY(cudaMemcpyAsync(dst, origins, 3 * n * f, cudaMemcpyHostToDevice, scene->stream));
+  CUDA_TRY(cudaMemcpyAsync(dst + 3 * n, directions, 3 * n * f, cudaMemcpyHostToDevice, scene->stream));
+  if (limits) CUDA_TRY(cudaMemcpyAsync(dst + 6 * n, limits, n * f, cudaMemcpyHostToDevice, scene->stream));
+}
+
+void OccludedOnDevice(MuonScene *scene, const QueryRays &rays, const float *max_distance, int64_t n, int32_t mode,
+                      uint8_t *occluded) {
+  for (int64_t i = 0; i < n; i += kQueryLaunch) {
+    const QueryRays q{rays.origin + rays.stride * i, rays.direction + rays.stride * i, rays.stride};
+    LaunchOccludedRays(scene->dev, q, max_distance + i, static_cast<int>(std::min(n - i, kQueryLaunch)), mode,
+                       occluded + i, scene->stream);
+  }
+  CUDA_TRY(cudaGetLastError());
+}
+
+}  // namespace
+
+int muon_gpu_intersect(MuonScene *scene, const MuonRay *rays, int64_t n, int32_t intersect_mode, MuonHit *hits) {
+  const int rc = CheckQuery(scene, rays && hits, n, intersect_mode);
+  if (rc != MUON_OK || n == 0) return rc;
   static_assert(sizeof(MuonRay) == 24 && sizeof(MuonHit) == 32, "ray/hit layout");
   try {
     CUDA_TRY(cudaSetDevice(scene->device));
@@ -1211,8 +1268,9 @@ int muon_gpu_intersect(MuonScene *scene, const MuonRay *rays, int64_t n, int32_t
     scene->ray_in.Ensure(n * sizeof(MuonRay));
     scene->ray_out.Ensure(n * sizeof(MuonHit));
     CUDA_TRY(cudaMemcpyAsync(scene->ray_in.ptr, rays, n * sizeof(MuonRay), cudaMemcpyHostToDevice, st));
-    LaunchIntersectRays(scene->dev, scene->ray_in.as<float>(), n, intersect_mode, scene->ray_out.as<float>(), st);
-    CUDA_TRY(cudaGetLastError());
+    float *r = scene->ray_in.as<float>(), *h = scene->ray_out.as<float>();
+    IntersectOnDevice(scene, QueryRays{r, r + 3, 6}, n, intersect_mode,
+                      QueryHits{h, reinterpret_cast<int32_t *>(h + 1), h + 2, h + 5, 8, 8});
     CUDA_TRY(cudaMemcpyAsync(hits, scene->ray_out.ptr, n * sizeof(MuonHit), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
   } catch (const CudaError &e) {
@@ -1221,13 +1279,49 @@ int muon_gpu_intersect(MuonScene *scene, const MuonRay *rays, int64_t n, int32_t
   return MUON_OK;
 }
 
+int muon_gpu_intersect_arrays(MuonScene *scene, const float *origins, const float *directions, int64_t n,
+                              int32_t intersect_mode, float *distance, int32_t *prim_id, float *position,
+                              float *normal) {
+  const int rc = CheckQuery(scene, origins && directions && distance && prim_id && position && normal, n, intersect_mode);
+  if (rc != MUON_OK || n == 0) return rc;
+  try {
+    CUDA_TRY(cudaSetDevice(scene->device));
+    cudaStream_t st = scene->stream;
+    const size_t f = sizeof(float);
+    scene->ray_in.Ensure(n * 6 * f);
+    scene->ray_out.Ensure(n * 8 * f);
+    float *o = scene->ray_in.as<float>(), *d = o + 3 * n;
+    float *dist = scene->ray_out.as<float>(), *id = dist + n, *pos = dist + 2 * n, *nrm = dist + 5 * n;
+    std::vector<float> stage(n <= kQueryStaged ? 8 * n : 0);
+    SendRays(scene, origins, directions, nullptr, n, stage.data());
+    IntersectOnDevice(scene, QueryRays{o, d, 3}, n, intersect_mode,
+                      QueryHits{dist, reinterpret_cast<int32_t *>(id), pos, nrm, 1, 3});
+    if (stage.empty()) {
+      CUDA_TRY(cudaMemcpyAsync(distance, dist, n * f, cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaMemcpyAsync(prim_id, id, n * f, cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaMemcpyAsync(position, pos, 3 * n * f, cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaMemcpyAsync(normal, nrm, 3 * n * f, cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaStreamSynchronize(st));
+    } else {
+      CUDA_TRY(cudaMemcpyAsync(stage.data(), dist, 8 * n * f, cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaStreamSynchronize(st));
+      std::memcpy(distance, stage.data(), n * f);
+      std::memcpy(prim_id, stage.data() + n, n * f);
+      std::memcpy(position, stage.data() + 2 * n, 3 * n * f);
+      std::memcpy(normal, stage.data() + 5 * n, 3 * n * f);
+    }
+  } catch (const CudaError &e) {
+    return FailCuda(e);
+  } catch (const std::bad_alloc &) {
+    return Fail(MUON_ERR_OOM, "host allocation failed");
+  }
+  return MUON_OK;
+}
+
 int muon_gpu_occluded(MuonScene *scene, const MuonRay *rays, const float *max_distance, int64_t n,
                       int32_t intersect_mode, uint8_t *occluded) {
-  if (!scene || (n > 0 && (!rays || !max_distance || !occluded)) || n < 0)
-    return Fail(MUON_ERR_INVALID_ARG, "bad argument");
-  if (intersect_mode < MUON_ISECT_FAST || intersect_mode > MUON_ISECT_EXACT)
-    return Fail(MUON_ERR_INVALID_ARG, "unknown intersect_mode");
-  if (n == 0) return MUON_OK;
+  const int rc = CheckQuery(scene, rays && max_distance && occluded, n, intersect_mode);
+  if (rc != MUON_OK || n == 0) return rc;
   try {
     CUDA_TRY(cudaSetDevice(scene->device));
     cudaStream_t st = scene->stream;
@@ -1236,13 +1330,36 @@ int muon_gpu_occluded(MuonScene *scene, const MuonRay *rays, const float *max_di
     scene->ray_out.Ensure(n);
     CUDA_TRY(cudaMemcpyAsync(scene->ray_in.ptr, rays, n * sizeof(MuonRay), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(scene->ray_aux.ptr, max_distance, n * sizeof(float), cudaMemcpyHostToDevice, st));
-    LaunchOccludedRays(scene->dev, scene->ray_in.as<float>(), scene->ray_aux.as<float>(), n, intersect_mode,
-                       scene->ray_out.as<uint8_t>(), st);
-    CUDA_TRY(cudaGetLastError());
+    const float *r = scene->ray_in.as<float>();
+    OccludedOnDevice(scene, QueryRays{r, r + 3, 6}, scene->ray_aux.as<float>(), n, intersect_mode,
+                     scene->ray_out.as<uint8_t>());
     CUDA_TRY(cudaMemcpyAsync(occluded, scene->ray_out.ptr, n, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
   } catch (const CudaError &e) {
     return FailCuda(e);
+  }
+  return MUON_OK;
+}
+
+int muon_gpu_occluded_arrays(MuonScene *scene, const float *origins, const float *directions, const float *max_distance,
+                             int64_t n, int32_t intersect_mode, uint8_t *occluded) {
+  const int rc = CheckQuery(scene, origins && directions && max_distance && occluded, n, intersect_mode);
+  if (rc != MUON_OK || n == 0) return rc;
+  try {
+    CUDA_TRY(cudaSetDevice(scene->device));
+    cudaStream_t st = scene->stream;
+    scene->ray_in.Ensure(n * 7 * sizeof(float));
+    scene->ray_out.Ensure(n);
+    std::vector<float> stage(n <= kQueryStaged ? 7 * n : 0);
+    SendRays(scene, origins, directions, max_distance, n, stage.data());
+    const float *o = scene->ray_in.as<float>();
+    OccludedOnDevice(scene, QueryRays{o, o + 3 * n, 3}, o + 6 * n, n, intersect_mode, scene->ray_out.as<uint8_t>());
+    CUDA_TRY(cudaMemcpyAsync(occluded, scene->ray_out.ptr, n, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+  } catch (const CudaError &e) {
+    return FailCuda(e);
+  } catch (const std::bad_alloc &) {
+    return Fail(MUON_ERR_OOM, "host allocation failed");
   }
   return MUON_OK;
 }

@@ -162,6 +162,10 @@ SIGNATURES = {
     "muon_gpu_intersect": (C.c_int, [C.c_void_p, C.POINTER(Ray), C.c_int64, C.c_int32, C.POINTER(Hit)]),
     "muon_gpu_occluded": (C.c_int, [C.c_void_p, C.POINTER(Ray), C.POINTER(C.c_float), C.c_int64, C.c_int32,
                                     C.POINTER(C.c_uint8)]),
+    "muon_gpu_intersect_arrays": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p,
+                                            C.c_void_p, C.c_void_p, C.c_void_p]),
+    "muon_gpu_occluded_arrays": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32,
+                                           C.c_void_p]),
     "muon_gpu_stats": (C.c_int, [C.c_void_p, C.POINTER(Stats)]),
     "muon_walk_rays": (C.c_int, [C.POINTER(SceneDesc), C.POINTER(Ray), C.POINTER(C.c_float), C.c_int64, C.c_int32,
                                  C.c_int32, C.POINTER(C.c_int32), C.POINTER(WalkCounts)]),
