@@ -162,7 +162,7 @@ void MergeScenes(MuonBatch *b, const std::vector<SceneView> &views) {
   }
   if (total_nodes > INT32_MAX || total_prims > INT32_MAX) throw CudaError{cudaErrorInvalidValue, "batch too large"};
   cudaStream_t st = b->stream;
-  b->nodes.Ensure(sizeof(BvhNode) * total_nodes);
+  b->nodes.Ensure(sizeof(DevNode) * total_nodes);
   b->prims.Ensure(sizeof(PrimRecord) * std::max<int64_t>(total_prims, 1));
   b->prims_obj.Ensure(sizeof(PrimRecord) * std::max<int64_t>(total_prims, 1));
   b->shade.Ensure(sizeof(ShadeRecord) * std::max<int64_t>(total_prims, 1));
@@ -170,8 +170,8 @@ void MergeScenes(MuonBatch *b, const std::vector<SceneView> &views) {
   b->smooth_obj.Ensure(any_smooth ? sizeof(F4) * 3 * total_prims : 16);
   // No primitives: a root whose first child link is empty ends every
   // traversal at once.
-  BvhNode empty{};
-  empty.d.x = empty.d.y = kEmptyLink;
+  DevNode empty{};
+  empty.child[0].link = empty.child[1].link = kEmptyLink;
   int32_t node_off = 0, prim_off = 0;
   for (const SceneView &v : views) {
     const SceneImage &im = *v.img;
@@ -189,10 +189,10 @@ void MergeScenes(MuonBatch *b, const std::vector<SceneView> &views) {
     b->cams.push_back(*v.cam);
     const int64_t nn = v.dev->num_nodes;
     if (nn == 0)
-      CUDA_TRY(cudaMemcpyAsync(b->nodes.as<BvhNode>() + node_off, &empty, sizeof(BvhNode), cudaMemcpyHostToDevice, st));
+      CUDA_TRY(cudaMemcpyAsync(b->nodes.as<DevNode>() + node_off, &empty, sizeof(DevNode), cudaMemcpyHostToDevice, st));
     const MergeOffsets off{node_off, prim_off, xf_off, mat_off, light_off};
     LaunchMergeScene(v.dev->nodes, nn, v.dev->prims, v.dev->prims_obj, v.dev->shade, v.dev->smooth_normals,
-                     v.dev->smooth_normals_obj, v.num_slots, off, b->nodes.as<BvhNode>(), b->prims.as<PrimRecord>(),
+                     v.dev->smooth_normals_obj, v.num_slots, off, b->nodes.as<DevNode>(), b->prims.as<PrimRecord>(),
                      b->prims_obj.as<PrimRecord>(), b->shade.as<ShadeRecord>(),
                      any_smooth ? b->smooth.as<F4>() : nullptr, any_smooth ? b->smooth_obj.as<F4>() : nullptr, st);
     CUDA_TRY(cudaGetLastError());
@@ -215,7 +215,7 @@ void MergeScenes(MuonBatch *b, const std::vector<SceneView> &views) {
   Upload(b->other_lights, other, st);
   DevScene &d = b->dev;
   d = DevScene{};
-  d.nodes = b->nodes.as<BvhNode>();
+  d.nodes = b->nodes.as<DevNode>();
   d.prims = b->prims.as<PrimRecord>();
   d.prims_obj = b->prims_obj.as<PrimRecord>();
   d.shade = b->shade.as<ShadeRecord>();

@@ -10,7 +10,10 @@
 //   d = (link0, link1, -, -)
 // A link >= 0 is an interior node index; a link < 0 is a leaf whose first
 // primitive record is ~link. Leaves end at the record flagged kPrimLast.
-// Node 0 is the root; an empty child slot has an inverted box.
+// Node 0 is the root; an empty child slot has an inverted box. That is the
+// form that the builders write and hosts read (BvhNode). The kernels' copy
+// (DevNode) holds the same words child by child, so that each child is one
+// 32-byte load and a lane may load either first.
 //
 // Primitive records (64 bytes, leaf order), world space:
 //   triangle: p0 = (a.xyz, dot(a,n)), p1 = (b.xyz, eps), p2 = (c.xyz, -),
@@ -52,6 +55,16 @@ struct alignas(16) BvhNode {
 };
 static_assert(sizeof(BvhNode) == 64, "BVH node must be 64 bytes");
 
+struct alignas(32) DevChild {
+  F4 xy;  // lo.x, hi.x, lo.y, hi.y
+  float lo_z, hi_z;
+  int32_t link, pad;
+};
+struct DevNode {
+  DevChild child[2];
+};
+static_assert(sizeof(DevNode) == sizeof(BvhNode), "nodes are converted in place");
+
 struct alignas(16) PrimRecord {
   F4 p0, p1, p2, p3;
 };
@@ -92,7 +105,7 @@ struct alignas(16) DevLight {
 
 // Pointers into one scene's device arrays (all leaf order where relevant).
 struct DevScene {
-  const BvhNode *nodes;
+  const DevNode *nodes;
   const PrimRecord *prims;      // world-space records (fast / watertight)
   const PrimRecord *prims_obj;  // object-space records (exact)
   const ShadeRecord *shade;

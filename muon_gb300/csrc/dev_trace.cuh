@@ -59,8 +59,9 @@ __device__ __forceinline__ float Min3(float a, float b, float c) {
 #endif
 }
 
-// BVH nodes and primitive records (64 bytes, 64-byte aligned) read with two
-// 256-bit loads instead of four 128-bit ones: half the load requests to L1.
+// Primitive records (64 bytes, 64-byte aligned) read with two 256-bit loads
+// instead of four 128-bit ones, as nodes are (TestChildren): half the load
+// requests to L1.
 #ifndef MUON_LD256
 #define MUON_LD256 1
 #endif
@@ -296,6 +297,55 @@ struct TraceCounters {
   uint32_t box_tests = 0, box_hits = 0, prim_tests = 0, prim_hits = 0;
 };
 
+// A node's two children as a lane tests them: A is the half it loads first.
+struct NodeHits {
+  bool hit_a, hit_b, b_first;  // b_first: B is visited before A where both are hit
+  int link_a, link_b;
+};
+
+__device__ __forceinline__ void LoadChild(const char *p, float4 &xy, float4 &z) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(xy.x), "=f"(xy.y), "=f"(xy.z), "=f"(xy.w), "=f"(z.x), "=f"(z.y), "=f"(z.z), "=f"(z.w)
+      : "l"(p));
+}
+
+// Tests both child boxes of a node. `odd`: load child 1 first.
+//
+// The lanes of a warp are at different nodes, and the walks of deep trees are
+// bound by L1's data banks. If every lane loads its node's first half and then
+// the second, the lanes of one load all want the same half of the banks; so
+// there the odd lanes begin with the other half. The halves are alike, so
+// nothing has to be moved, and the visiting order is the same: the nearer
+// child first, child 0 at equal distances. On the dense mesh (512 x 512, 16
+// samples) bank conflicts fall by 45% and the walks take 71.5 ms instead of
+// 74.7. The walks of small trees are bound by latency and issue; the few
+// instructions it costs made them 2 to 7% slower (Cornell box, sphere
+// field): they pass false.
+__device__ __forceinline__ NodeHits TestChildren(const DevNode *node, const RayPre &r, float tmax, bool odd) {
+  const char *pa = reinterpret_cast<const char *>(node) + (odd ? 32 : 0);
+  float4 axy, az, bxy, bz;
+  LoadChild(pa, axy, az);
+  LoadChild(reinterpret_cast<const char *>(reinterpret_cast<uintptr_t>(pa) ^ 32), bxy, bz);
+  const float alox = axy.x * r.idir.x - r.ood.x, ahix = axy.y * r.idir.x - r.ood.x;
+  const float aloy = axy.z * r.idir.y - r.ood.y, ahiy = axy.w * r.idir.y - r.ood.y;
+  const float aloz = az.x * r.idir.z - r.ood.z, ahiz = az.y * r.idir.z - r.ood.z;
+  const float blox = bxy.x * r.idir.x - r.ood.x, bhix = bxy.y * r.idir.x - r.ood.x;
+  const float bloy = bxy.z * r.idir.y - r.ood.y, bhiy = bxy.w * r.idir.y - r.ood.y;
+  const float bloz = bz.x * r.idir.z - r.ood.z, bhiz = bz.y * r.idir.z - r.ood.z;
+  const float amin = Max3(fminf(alox, ahix), fminf(aloy, ahiy), fmaxf(fminf(aloz, ahiz), 0.0f));
+  const float amax = Min3(fmaxf(alox, ahix), fmaxf(aloy, ahiy), fminf(fmaxf(aloz, ahiz), tmax));
+  const float bmin = Max3(fminf(blox, bhix), fminf(bloy, bhiy), fmaxf(fminf(bloz, bhiz), 0.0f));
+  const float bmax = Min3(fmaxf(blox, bhix), fmaxf(bloy, bhiy), fminf(fmaxf(bloz, bhiz), tmax));
+  NodeHits c;
+  c.hit_a = amin <= amax;
+  c.hit_b = bmin <= bmax;
+  // neither is negative, so their bits compare as the values do
+  c.b_first = __float_as_int(bmin) < __float_as_int(amin) + (odd ? 1 : 0);
+  c.link_a = __float_as_int(az.z);
+  c.link_b = __float_as_int(bz.z);
+  return c;
+}
+
 // Closest hit (kAnyHit = false) or first hit (kAnyHit = true) with
 // 0 < t < tmax. Returns the leaf slot of the primitive hit, or -1; *t_hit
 // receives its distance. A stack overflow sets *overflow.
@@ -312,37 +362,24 @@ __device__ __forceinline__ int Trace(const DevScene &s, float3 o, float3 d, floa
     // Interior nodes: test both child boxes, descend into the nearer hit child
     // and defer the farther one.
     while (node >= 0) {
-      float4 n0, n1, n2, n3f;
-      Load64B(s.nodes + node, n0, n1, n2, n3f);
-      const int4 n3 = make_int4(__float_as_int(n3f.x), __float_as_int(n3f.y), 0, 0);
-      float c0lox = n0.x * r.idir.x - r.ood.x, c0hix = n0.y * r.idir.x - r.ood.x;
-      float c0loy = n0.z * r.idir.y - r.ood.y, c0hiy = n0.w * r.idir.y - r.ood.y;
-      float c0loz = n2.x * r.idir.z - r.ood.z, c0hiz = n2.y * r.idir.z - r.ood.z;
-      float c1lox = n1.x * r.idir.x - r.ood.x, c1hix = n1.y * r.idir.x - r.ood.x;
-      float c1loy = n1.z * r.idir.y - r.ood.y, c1hiy = n1.w * r.idir.y - r.ood.y;
-      float c1loz = n2.z * r.idir.z - r.ood.z, c1hiz = n2.w * r.idir.z - r.ood.z;
-      float c0min = Max3(fminf(c0lox, c0hix), fminf(c0loy, c0hiy), fmaxf(fminf(c0loz, c0hiz), 0.0f));
-      float c0max = Min3(fmaxf(c0lox, c0hix), fmaxf(c0loy, c0hiy), fminf(fmaxf(c0loz, c0hiz), tmax));
-      float c1min = Max3(fminf(c1lox, c1hix), fminf(c1loy, c1hiy), fmaxf(fminf(c1loz, c1hiz), 0.0f));
-      float c1max = Min3(fmaxf(c1lox, c1hix), fmaxf(c1loy, c1hiy), fminf(fmaxf(c1loz, c1hiz), tmax));
-      bool h0 = c0min <= c0max, h1 = c1min <= c1max;
+      const NodeHits c = TestChildren(s.nodes + node, r, tmax, false);
       if (kStats) {
         cnt->box_tests += 2;
-        cnt->box_hits += (int)h0 + (int)h1;
+        cnt->box_hits += (int)c.hit_a + (int)c.hit_b;
       }
-      if (!h0 && !h1) {
+      if (!c.hit_a && !c.hit_b) {
         if (sp == 0) {
           node = kEmptyLink;
           break;
         }
         node = stack[--sp];
       } else {
-        int near = h0 ? n3.x : n3.y;
-        if (h0 && h1) {
-          int far = n3.y;
-          if (c1min < c0min) {
-            near = n3.y;
-            far = n3.x;
+        int near = c.hit_a ? c.link_a : c.link_b;
+        if (c.hit_a && c.hit_b) {
+          int far = c.link_b;
+          if (c.b_first) {
+            near = c.link_b;
+            far = c.link_a;
           }
           if (sp < kStackSize) {
             stack[sp++] = far;
@@ -442,37 +479,24 @@ __device__ __forceinline__ bool TravRun(const DevScene &s, RayPre &r, TravState 
   if (s.num_nodes == 0) return true;
   while (true) {
     while (t.node >= 0) {
-      float4 n0, n1, n2, n3f;
-      Load64B(s.nodes + t.node, n0, n1, n2, n3f);
-      const int4 n3 = make_int4(__float_as_int(n3f.x), __float_as_int(n3f.y), 0, 0);
-      float c0lox = n0.x * r.idir.x - r.ood.x, c0hix = n0.y * r.idir.x - r.ood.x;
-      float c0loy = n0.z * r.idir.y - r.ood.y, c0hiy = n0.w * r.idir.y - r.ood.y;
-      float c0loz = n2.x * r.idir.z - r.ood.z, c0hiz = n2.y * r.idir.z - r.ood.z;
-      float c1lox = n1.x * r.idir.x - r.ood.x, c1hix = n1.y * r.idir.x - r.ood.x;
-      float c1loy = n1.z * r.idir.y - r.ood.y, c1hiy = n1.w * r.idir.y - r.ood.y;
-      float c1loz = n2.z * r.idir.z - r.ood.z, c1hiz = n2.w * r.idir.z - r.ood.z;
-      float c0min = Max3(fminf(c0lox, c0hix), fminf(c0loy, c0hiy), fmaxf(fminf(c0loz, c0hiz), 0.0f));
-      float c0max = Min3(fmaxf(c0lox, c0hix), fmaxf(c0loy, c0hiy), fminf(fmaxf(c0loz, c0hiz), t.tmax));
-      float c1min = Max3(fminf(c1lox, c1hix), fminf(c1loy, c1hiy), fmaxf(fminf(c1loz, c1hiz), 0.0f));
-      float c1max = Min3(fmaxf(c1lox, c1hix), fmaxf(c1loy, c1hiy), fminf(fmaxf(c1loz, c1hiz), t.tmax));
-      bool h0 = c0min <= c0max, h1 = c1min <= c1max;
+      const NodeHits c = TestChildren(s.nodes + t.node, r, t.tmax, false);
       if (kStats) {
         cnt->box_tests += 2;
-        cnt->box_hits += (int)h0 + (int)h1;
+        cnt->box_hits += (int)c.hit_a + (int)c.hit_b;
       }
-      if (!h0 && !h1) {
+      if (!c.hit_a && !c.hit_b) {
         if (t.sp == 0) {
           t.node = kEmptyLink;
           break;
         }
         t.node = StackPop(t);
       } else {
-        int near = h0 ? n3.x : n3.y;
-        if (h0 && h1) {
-          int far = n3.y;
-          if (c1min < c0min) {
-            near = n3.y;
-            far = n3.x;
+        int near = c.hit_a ? c.link_a : c.link_b;
+        if (c.hit_a && c.hit_b) {
+          int far = c.link_b;
+          if (c.b_first) {
+            near = c.link_b;
+            far = c.link_a;
           }
           if (t.sp < kStackSize) StackPush(t, far);
           else *overflow = true;
@@ -524,38 +548,26 @@ template <bool kAnyHit, bool kStats, int kTriTest, int kMinDescend>
 __device__ __forceinline__ bool TravRunSpeculative(const DevScene &s, RayPre &r, TravState &t, TraceCounters *cnt,
                                                    bool *overflow, int min_active) {
   if (s.num_nodes == 0) return true;
+  const bool odd = kMinDescend > 0 && (threadIdx.x & 1);  // see TestChildren
   auto next = [&] { t.node = t.sp == 0 ? kEmptyLink : StackPop(t); };
   const PrimRecord *recs = kTriTest == MUON_ISECT_EXACT ? s.prims_obj : s.prims;
   while (true) {
     int leaf = 0;  // postponed leaf link (leaf links are negative; 0 = none)
     while (t.node >= 0) {
-      float4 n0, n1, n2, n3f;
-      Load64B(s.nodes + t.node, n0, n1, n2, n3f);
-      const int4 n3 = make_int4(__float_as_int(n3f.x), __float_as_int(n3f.y), 0, 0);
-      float c0lox = n0.x * r.idir.x - r.ood.x, c0hix = n0.y * r.idir.x - r.ood.x;
-      float c0loy = n0.z * r.idir.y - r.ood.y, c0hiy = n0.w * r.idir.y - r.ood.y;
-      float c0loz = n2.x * r.idir.z - r.ood.z, c0hiz = n2.y * r.idir.z - r.ood.z;
-      float c1lox = n1.x * r.idir.x - r.ood.x, c1hix = n1.y * r.idir.x - r.ood.x;
-      float c1loy = n1.z * r.idir.y - r.ood.y, c1hiy = n1.w * r.idir.y - r.ood.y;
-      float c1loz = n2.z * r.idir.z - r.ood.z, c1hiz = n2.w * r.idir.z - r.ood.z;
-      float c0min = Max3(fminf(c0lox, c0hix), fminf(c0loy, c0hiy), fmaxf(fminf(c0loz, c0hiz), 0.0f));
-      float c0max = Min3(fmaxf(c0lox, c0hix), fmaxf(c0loy, c0hiy), fminf(fmaxf(c0loz, c0hiz), t.tmax));
-      float c1min = Max3(fminf(c1lox, c1hix), fminf(c1loy, c1hiy), fmaxf(fminf(c1loz, c1hiz), 0.0f));
-      float c1max = Min3(fmaxf(c1lox, c1hix), fmaxf(c1loy, c1hiy), fminf(fmaxf(c1loz, c1hiz), t.tmax));
-      bool h0 = c0min <= c0max, h1 = c1min <= c1max;
+      const NodeHits c = TestChildren(s.nodes + t.node, r, t.tmax, odd);
       if (kStats) {
         cnt->box_tests += 2;
-        cnt->box_hits += (int)h0 + (int)h1;
+        cnt->box_hits += (int)c.hit_a + (int)c.hit_b;
       }
-      if (!h0 && !h1) {
+      if (!c.hit_a && !c.hit_b) {
         next();
       } else {
-        int near = h0 ? n3.x : n3.y;
-        if (h0 && h1) {
-          int far = n3.y;
-          if (c1min < c0min) {
-            near = n3.y;
-            far = n3.x;
+        int near = c.hit_a ? c.link_a : c.link_b;
+        if (c.hit_a && c.hit_b) {
+          int far = c.link_b;
+          if (c.b_first) {
+            near = c.link_b;
+            far = c.link_a;
           }
           if (t.sp < kStackSize) StackPush(t, far);
           else *overflow = true;

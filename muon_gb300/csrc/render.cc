@@ -1106,8 +1106,10 @@ int muon_gpu_scene_create(const MuonSceneDesc *desc, MuonScene **out) {
     Upload(sc->light_tris, lt, st);
     Upload(sc->light_tris_obj, lt_obj, st);
     Upload(sc->light_tri_ok, lt_ok, st);
+    LaunchNodeLayout(sc->nodes.as<BvhNode>(), static_cast<int64_t>(im.nodes.size()), st);
+    CUDA_TRY(cudaGetLastError());
     DevScene &d = sc->dev;
-    d.nodes = sc->nodes.as<BvhNode>();
+    d.nodes = sc->nodes.as<DevNode>();
     d.prims = sc->prims.as<PrimRecord>();
     d.prims_obj = sc->prims_obj.as<PrimRecord>();
     d.shade = sc->shade.as<ShadeRecord>();

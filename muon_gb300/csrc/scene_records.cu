@@ -57,12 +57,21 @@ __device__ __forceinline__ int32_t ShiftLink(int32_t link, int32_t node_off, int
   return ~(~link + prim_off);
 }
 
-__global__ void MergeNodesKernel(const BvhNode *in, int64_t n, MergeOffsets off, BvhNode *out) {
+__global__ void NodeLayoutKernel(BvhNode *nodes, int64_t n) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
   if (i >= n) return;
-  BvhNode nd = in[i];
-  nd.d.x = ShiftLink(nd.d.x, off.node_off, off.prim_off);
-  nd.d.y = ShiftLink(nd.d.y, off.node_off, off.prim_off);
+  const BvhNode nd = nodes[i];
+  DevNode out;
+  out.child[0] = DevChild{nd.a, nd.c.x, nd.c.y, nd.d.x, 0};
+  out.child[1] = DevChild{nd.b, nd.c.z, nd.c.w, nd.d.y, 0};
+  reinterpret_cast<DevNode *>(nodes)[i] = out;
+}
+
+__global__ void MergeNodesKernel(const DevNode *in, int64_t n, MergeOffsets off, DevNode *out) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  if (i >= n) return;
+  DevNode nd = in[i];
+  for (DevChild &c : nd.child) c.link = ShiftLink(c.link, off.node_off, off.prim_off);
   out[off.node_off + i] = nd;
 }
 
@@ -97,14 +106,18 @@ __global__ void MergePrimsKernel(const PrimRecord *prims_in, const PrimRecord *o
 
 }  // namespace
 
-void LaunchMergeScene(const BvhNode *nodes_in, int64_t num_nodes, const PrimRecord *prims_in,
+void LaunchMergeScene(const DevNode *nodes_in, int64_t num_nodes, const PrimRecord *prims_in,
                       const PrimRecord *obj_in, const ShadeRecord *shade_in, const F4 *sn_in, const F4 *sno_in,
-                      int64_t num_prims, MergeOffsets off, BvhNode *nodes_out, PrimRecord *prims_out,
+                      int64_t num_prims, MergeOffsets off, DevNode *nodes_out, PrimRecord *prims_out,
                       PrimRecord *obj_out, ShadeRecord *shade_out, F4 *sn_out, F4 *sno_out, cudaStream_t st) {
   if (num_nodes > 0) MergeNodesKernel<<<Grid(num_nodes), kThreads, 0, st>>>(nodes_in, num_nodes, off, nodes_out);
   if (num_prims > 0)
     MergePrimsKernel<<<Grid(num_prims), kThreads, 0, st>>>(prims_in, obj_in, shade_in, sn_in, sno_in, num_prims, off,
                                                           prims_out, obj_out, shade_out, sn_out, sno_out);
+}
+
+void LaunchNodeLayout(BvhNode *nodes, int64_t n, cudaStream_t st) {
+  if (n > 0) NodeLayoutKernel<<<Grid(n), kThreads, 0, st>>>(nodes, n);
 }
 
 size_t HittableScanBytes(int64_t n) {
