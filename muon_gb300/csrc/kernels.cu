@@ -345,9 +345,11 @@ constexpr int kRefillThreshold = MUON_REFILL_THRESHOLD;
 // at least kDeepNodes nodes. Extend + occlude ms of dense-mesh frames without and
 // with, by nodes: 512x512x16 6.70 / 6.72 (1,737), 7.32 / 7.21 (3,959), 8.02 / 7.91
 // (12,878), 12.20 / 11.43 (52,694), 13.39 / 12.44 (195,485); 1024x1024x16 84.2 /
-// 74.4 (773,807); there 8, 12 and 20 lanes give 78.1, 75.6 and 74.6. Shallow trees
-// lose, their lanes reach leaves together: sphere field (448 nodes) 1.99 / 2.17,
-// Cornell box 0.80 / 0.89. So do batches, whose wavefronts mix trees (batch.cc).
+// 74.4 (773,807). With the halves loaded in turn (TestChildren) the last is 71.5;
+// there 12, 14, 18 and 20 lanes give 73.4, 72.5, 71.3 and 71.1, but 18 and 20 cost
+// the 12,878-node mesh 1 to 3%. Shallow trees lose, their lanes reach leaves
+// together: sphere field (448 nodes) 1.99 / 2.17, Cornell box 0.80 / 0.89. So do
+// batches, whose wavefronts mix trees (batch.cc).
 constexpr int kDeepMinDescend = 16;
 constexpr int kDeepNodes = 8192;
 // Minimum resident blocks per SM the traversal kernels are compiled for.
