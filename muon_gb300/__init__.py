@@ -147,8 +147,15 @@ class FilmResult:
 
 
 def _vectors(a, n: int) -> np.ndarray:
-    """n vectors as contiguous float32 (n, 3), broadcast like an assignment."""
-    return np.ascontiguousarray(np.broadcast_to(np.asarray(a), (n, 3)), dtype=np.float32)
+    """n vectors as contiguous float32 (n, 3): `a` itself if it is that already,
+    else what an assignment makes of it (which also drops leading axes of
+    length 1, unlike np.broadcast_to)."""
+    if isinstance(a, np.ndarray) and a.shape == (n, 3) and a.dtype == np.float32 and a.flags.c_contiguous \
+            and a.flags.aligned:
+        return a
+    v = np.empty((n, 3), dtype=np.float32)
+    v[...] = a
+    return v
 
 
 # Below this many primitives the host builds the SAH tree faster than the
