@@ -158,6 +158,16 @@ def _vectors(a, n: int) -> np.ndarray:
     return v
 
 
+def _limits(a, n: int) -> np.ndarray:
+    """At least n limits as contiguous float32; a single one serves all rays."""
+    v = np.ascontiguousarray(a, dtype=np.float32)
+    if v.size == 1:
+        return np.full(n, v.reshape(-1)[0])
+    if v.size < n:
+        raise ValueError(f"{v.size} limits for {n} rays")
+    return v
+
+
 # Below this many primitives the host builds the SAH tree faster than the
 # device's launches and synchronisations (measured on a GB300: 36 primitives
 # 0.20 ms on the host vs 0.39 ms on the device; 516 primitives 1.04 vs 0.55 ms).
@@ -263,10 +273,11 @@ class Scene:
 
     def occluded(self, origins: np.ndarray, directions: np.ndarray, max_distance: np.ndarray,
                  intersect_mode: int = native.ISECT_EXACT) -> np.ndarray:
-        """Any hit closer than max_distance (Structure::HasIntersection)."""
+        """Any hit closer than max_distance, a limit per ray or one for all
+        (Structure::HasIntersection)."""
         n = len(origins)
         o, d = _vectors(origins, n), _vectors(directions, n)
-        md = np.ascontiguousarray(max_distance, dtype=np.float32)
+        md = _limits(max_distance, n)
         out = np.empty(n, dtype=bool)
         check(load().muon_gpu_occluded_arrays(self._h, o.ctypes.data, d.ctypes.data, md.ctypes.data, n, intersect_mode,
                                               out.ctypes.data))

@@ -58,3 +58,26 @@ def test_vectors_convert_like_an_assignment(recorded, n):
             scene.intersect(o, bad)
         with pytest.raises(ValueError):
             scene.occluded(o, bad, np.ones(n))
+
+
+@pytest.mark.parametrize("n", [2, 5])
+def test_limits_hold_a_value_for_every_ray(recorded, n):
+    """Fewer limits than rays were read past their end; one limit serves all
+    rays, and of more than n values the first n count, as before."""
+    scene, recorder = recorded
+    rng = np.random.default_rng(n)
+    o, d = rng.normal(size=(2, n, 3)).astype(np.float32)
+    for short in (np.ones(n - 1), np.ones(0), []):
+        if np.size(short) != 1:
+            with pytest.raises(ValueError):
+                scene.occluded(o, d, short)
+    for one in (1.5, np.float32(1.5), [1.5], np.full((1, 1), 1.5)):
+        scene.occluded(o, d, one)
+        assert np.array_equal(recorder.limits, np.full(n, 1.5, dtype=np.float32))
+    far = rng.uniform(0, 2, 2 * n).astype(np.float32)
+    for many in (far[:n], far[:n, None], far[:n].tolist(), far[:n].astype(np.float64), far, far.reshape(2, n)):
+        scene.occluded(o, d, many)
+        assert np.array_equal(recorder.limits, far[:n])
+    scene.occluded(o, d, far[::2])
+    assert np.array_equal(recorder.limits, far[::2])
+    assert scene.occluded(np.zeros((0, 3)), np.zeros((0, 3)), []).shape == (0,)
