@@ -198,7 +198,7 @@ typedef struct MuonRenderParams {
   int32_t intersect_mode; /* MUON_ISECT_* */
   int32_t wave_paths;    /* paths per wavefront (0 = 2^24); a render     */
                          /* keeps two wavefronts in flight, each with  */
-                         /* about 200 + 36 x shadow slots bytes a path */
+                         /* about 210 + 36 x shadow slots bytes a path */
   uint32_t flags;        /* MUON_RENDER_*                               */
   int32_t pad;
 } MuonRenderParams;

@@ -272,7 +272,7 @@ void RenderBatch(MuonBatch *b, const MuonRenderParams *params, double *const *d_
 
   // Wave plan: scenes in schedule order, cut into segments that fill waves.
   int64_t budget = b->wave_paths > 0 ? b->wave_paths : kBatchDefaultWavePaths;
-  const int64_t per_path = 200 + 36 * static_cast<int64_t>(std::max(S, 1));
+  const int64_t per_path = WorkBytesPerPath(S, 2);
   budget = std::max<int64_t>(1, std::min<int64_t>({budget, (int64_t(8) << 30) / per_path, int64_t(kMaxWavePaths)}));
   std::vector<BatchSeg> segs;
   std::vector<WavePlan> waves;

@@ -156,9 +156,10 @@ BouncePlan PlanBounces(const MuonRenderParams &p, const ShadeParams &sp);
 cudaError_t NoAllocPrepare();
 
 // Bytes of per-wavefront path state per path with `slots` shadow slots (the
-// arrays of PathBuffers, unpadded).
-inline int64_t WorkBytesPerPath(int slots) {
-  return 8 * 16 /* ray_o, ray_d, tp, rad (double-buffered) */ + 8 /* hits */ + 4 /* link */ +
+// arrays of PathBuffers, unpadded). hit_sets: arrays of hits and links, two
+// where bounces overlap.
+inline int64_t WorkBytesPerPath(int slots, int hit_sets) {
+  return 8 * 16 /* ray_o, ray_d, tp, rad (double-buffered) */ + hit_sets * (8 + 4) /* hits, link */ +
          16 /* final_rad */ + 16 /* org */ + int64_t(kNumClasses) * 4 /* order */ +
          int64_t(std::max(slots, 1)) * (16 + 16 + 4) /* contrib, slot_dir, shq */;
 }

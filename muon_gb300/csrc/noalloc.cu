@@ -102,7 +102,7 @@ size_t Carve(unsigned char *base, int64_t paths, int slots, int bounces, PathBuf
 
 // Largest multiple of 256 paths whose arrays fit the buffer (0 if none).
 int64_t Capacity(int slots, int bounces) {
-  int64_t lo = 0, hi = static_cast<int64_t>(kScratchBytes / WorkBytesPerPath(slots)) / 256 + 1;
+  int64_t lo = 0, hi = static_cast<int64_t>(kScratchBytes / WorkBytesPerPath(slots, 1)) / 256 + 1;
   while (lo + 1 < hi) {  // Carve(lo * 256) fits, Carve(hi * 256) does not
     const int64_t mid = (lo + hi) / 2;
     if (Carve(nullptr, mid * 256, slots, bounces, nullptr, nullptr) <= kScratchBytes) lo = mid;

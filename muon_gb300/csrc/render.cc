@@ -622,7 +622,7 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   const int spp = p.pixel_samples;
   int64_t budget = p.wave_paths > 0 ? p.wave_paths : kDefaultWavePaths;
   // Keep per-wave path state within ~8 GiB.
-  budget = std::max<int64_t>(1, std::min<int64_t>(budget, (int64_t(8) << 30) / WorkBytesPerPath(slots)));
+  budget = std::max<int64_t>(1, std::min<int64_t>(budget, (int64_t(8) << 30) / WorkBytesPerPath(slots, 2)));
   budget = std::min<int64_t>(budget, kMaxWavePaths);
   const BouncePlan bp = PlanBounces(p, sp);
   const bool traces = bp.traces, bounded = bp.bounded;
