@@ -1563,6 +1563,18 @@ void WithMode(int mode, F &&f) {
   else f(std::integral_constant<int, MUON_ISECT_FAST>());
 }
 
+// Calls f(std::bool_constant<counted>, std::bool_constant<deep>) for the variant of
+// the traversal kernels that a tree of `tree_nodes` nodes takes. Counted renders
+// take the same one: their counters are of the walk that runs without them.
+template <class F>
+void WithVariant(bool counted, int tree_nodes, F &&f) {
+  const bool deep = tree_nodes >= kDeepNodes;
+  if (counted && deep) f(std::true_type(), std::true_type());
+  else if (counted) f(std::true_type(), std::false_type());
+  else if (deep) f(std::false_type(), std::true_type());
+  else f(std::false_type(), std::false_type());
+}
+
 // ---- measurement ---------------------------------------------------------------
 // A sample of one bounce's traversal queue, copied for the host walk that
 // counts traversal work: kind 0 the closest-hit queue, kind 1 the shadow
@@ -1661,9 +1673,9 @@ void LaunchExtend(const DevScene &s, const PathBuffers &b, WaveCounters wc, int 
   WithMode(isect, [&](auto m) {
     constexpr int M = decltype(m)::value;
     const unsigned g = TraversalBlocks(bound);
-    if (stats) ExtendKernel<true, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
-    else if (tree_nodes >= kDeepNodes) ExtendKernel<false, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
-    else ExtendKernel<false, M, false><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
+    WithVariant(stats, tree_nodes, [&](auto counted, auto deep) {
+      ExtendKernel<decltype(counted)::value, M, decltype(deep)::value><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
+    });
   });
   if (MUON_STABLE_CLASSES && classes) {
     const int64_t segs = (static_cast<int64_t>(bound) + kClassTile - 1) / kClassTile;
@@ -1706,9 +1718,9 @@ void LaunchOcclude(const DevScene &s, const PathBuffers &b, WaveCounters wc, int
   WithMode(isect, [&](auto m) {
     constexpr int M = decltype(m)::value;
     const unsigned g = TraversalBlocks(bound);
-    if (stats) OccludeKernel<true, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
-    else if (tree_nodes >= kDeepNodes) OccludeKernel<false, M, true><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
-    else OccludeKernel<false, M, false><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
+    WithVariant(stats, tree_nodes, [&](auto counted, auto deep) {
+      OccludeKernel<decltype(counted)::value, M, decltype(deep)::value><<<g, kBlock, 0, st>>>(s, b, wc, bounce, slots);
+    });
   });
 }
 
