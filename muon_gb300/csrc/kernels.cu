@@ -1673,7 +1673,11 @@ void LaunchExtend(const DevScene &s, const PathBuffers &b, WaveCounters wc, int 
   WithMode(isect, [&](auto m) {
     constexpr int M = decltype(m)::value;
     const unsigned g = TraversalBlocks(bound);
-    WithVariant(stats, tree_nodes, [&](auto counted, auto deep) {
+    // Previews trace camera rays alone, whose lanes walk the same nodes together:
+    // there the deep trees' variant was slower than the full descent (normals of
+    // 270 x 270, us, with it / without: 14,948 nodes 125 / 102, 52,641 nodes
+    // 159 / 136, 773,807 nodes 152 / 125; 1024 x 1024: 186 / 174, 235 / 230, 230 / 219).
+    WithVariant(stats, classes ? tree_nodes : 0, [&](auto counted, auto deep) {
       ExtendKernel<decltype(counted)::value, M, decltype(deep)::value><<<g, kBlock, 0, st>>>(s, b, wc, bounce);
     });
   });

@@ -137,7 +137,8 @@ void SetTraversalGrid(int sms);
 void LaunchCamera(const DevCamera &cam, const WaveInfo &w, const PathBuffers &b, WaveCounters wc, cudaStream_t st);
 // tree_nodes: nodes of the scene's BVH, which picks the traversal kernels'
 // variant (0 for a batch). classes: build the class lists (which the path
-// tracer's shading reads and the preview integrators' does not).
+// tracer's shading reads and the preview integrators', whose camera rays take
+// the full descent in every tree, does not).
 void LaunchExtend(const DevScene &s, const PathBuffers &b, WaveCounters wc, int bounce, int bound, int isect,
                   bool stats, int tree_nodes, bool classes, cudaStream_t st);
 void LaunchShadeDebug(const DevScene &s, const PathBuffers &b, WaveCounters wc, int integrator, int bound, int isect,
