@@ -30,6 +30,8 @@
 
 #include <stdint.h>
 
+#include "mmath.h"
+
 namespace muon_gpu {
 
 constexpr uint32_t kPrimSphere = 1u;   // record is a sphere (else triangle)
@@ -64,6 +66,9 @@ struct DevNode {
   DevChild child[2];
 };
 static_assert(sizeof(DevNode) == sizeof(BvhNode), "nodes are converted in place");
+MM_HD DevNode ToDevNode(const BvhNode &n) {
+  return DevNode{{DevChild{n.a, n.c.x, n.c.y, n.d.x, 0}, DevChild{n.b, n.c.z, n.c.w, n.d.y, 0}}};
+}
 
 struct alignas(16) PrimRecord {
   F4 p0, p1, p2, p3;

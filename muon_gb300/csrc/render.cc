@@ -34,6 +34,11 @@ namespace {
 constexpr int kDefaultWavePaths = 1 << 24;
 constexpr int kMaxBounces = 256;  // hard cap for unbounded depth without Russian roulette
 constexpr int kMaxEventPairs = 16384;
+// Nodes of a host-built tree up to which the host brings them into the kernels'
+// form: a kernel behind the copies was waited for (scenes of 36 / 28 primitives
+// open in 188 / 199 us so, in 212 / 216 with it; 5 ms and more of host build hide
+// it for larger trees).
+constexpr size_t kHostLayoutNodes = 4096;
 
 }  // namespace
 
@@ -405,10 +410,16 @@ int BuildBvhOnGpu(MuonScene *sc, int builder, int max_leaf, cudaStream_t st, con
   CUDA_TRY(cudaGetLastError());
   im.nodes.resize(nn);
   CUDA_TRY(cudaMemcpyAsync(im.nodes.data(), sc->nodes.ptr, sizeof(BvhNode) * nn, cudaMemcpyDeviceToHost, st));
+  // beside the host's work that follows its copy of the nodes
+  auto layout = [&] {
+    LaunchNodeLayout(sc->nodes.as<BvhNode>(), nn, st);
+    CUDA_TRY(cudaGetLastError());
+  };
   if (sah) {
     // the records stay on the device until a host reader asks for them
     // (SyncSceneImage); the scene box and the node count come from the nodes
     CUDA_TRY(cudaStreamSynchronize(st));
+    layout();
     im.boxes.clear();
     im.boxes.shrink_to_fit();
     sc->host_records_stale = true;
@@ -432,6 +443,7 @@ int BuildBvhOnGpu(MuonScene *sc, int builder, int max_leaf, cudaStream_t st, con
                              cudaMemcpyDeviceToHost, st));
   }
   CUDA_TRY(cudaStreamSynchronize(st));
+  layout();
   im.boxes.clear();
   im.boxes.shrink_to_fit();
   for (int slot = 0; slot < n; ++slot) im.leaf_of_prim_id[im.shade[slot].s1.y] = slot;
@@ -1081,6 +1093,7 @@ int muon_gpu_scene_create(const MuonSceneDesc *desc, MuonScene **out) {
     CUDA_TRY(cudaStreamCreateWithFlags(&sc->stream, cudaStreamNonBlocking));
     cudaStream_t st = sc->stream;
     const SceneImage &im = sc->img;
+    std::vector<DevNode> dev_nodes;
     if (device_records || (gpu_bvh && !im.prims.empty())) {
       const int rc = BuildBvhOnGpu(sc.get(), desc->builder, desc->max_leaf_size > 0 ? desc->max_leaf_size : 4, st,
                                    device_records ? desc : nullptr);
@@ -1088,7 +1101,15 @@ int muon_gpu_scene_create(const MuonSceneDesc *desc, MuonScene **out) {
       if (sc->img.bvh.max_depth >= 60) return Fail(MUON_ERR_INVALID_ARG, "BVH too deep for the traversal stack");
     } else {
       sc->num_slots = static_cast<int64_t>(im.prims.size());
-      UploadPooled(sc->nodes, im.nodes, st, sc->device);
+      if (im.nodes.size() <= kHostLayoutNodes) {
+        dev_nodes.reserve(im.nodes.size());
+        for (const BvhNode &n : im.nodes) dev_nodes.push_back(ToDevNode(n));
+        UploadPooled(sc->nodes, dev_nodes, st, sc->device);
+      } else {
+        UploadPooled(sc->nodes, im.nodes, st, sc->device);
+        LaunchNodeLayout(sc->nodes.as<BvhNode>(), static_cast<int64_t>(im.nodes.size()), st);
+        CUDA_TRY(cudaGetLastError());
+      }
       UploadPooled(sc->prims, im.prims, st, sc->device);
       UploadPooled(sc->prims_obj, im.prims_obj, st, sc->device);
       UploadPooled(sc->shade, im.shade, st, sc->device);
@@ -1106,8 +1127,6 @@ int muon_gpu_scene_create(const MuonSceneDesc *desc, MuonScene **out) {
     Upload(sc->light_tris, lt, st);
     Upload(sc->light_tris_obj, lt_obj, st);
     Upload(sc->light_tri_ok, lt_ok, st);
-    LaunchNodeLayout(sc->nodes.as<BvhNode>(), static_cast<int64_t>(im.nodes.size()), st);
-    CUDA_TRY(cudaGetLastError());
     DevScene &d = sc->dev;
     d.nodes = sc->nodes.as<DevNode>();
     d.prims = sc->prims.as<PrimRecord>();

@@ -60,11 +60,7 @@ __device__ __forceinline__ int32_t ShiftLink(int32_t link, int32_t node_off, int
 __global__ void NodeLayoutKernel(BvhNode *nodes, int64_t n) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
   if (i >= n) return;
-  const BvhNode nd = nodes[i];
-  DevNode out;
-  out.child[0] = DevChild{nd.a, nd.c.x, nd.c.y, nd.d.x, 0};
-  out.child[1] = DevChild{nd.b, nd.c.z, nd.c.w, nd.d.y, 0};
-  reinterpret_cast<DevNode *>(nodes)[i] = out;
+  reinterpret_cast<DevNode *>(nodes)[i] = ToDevNode(nodes[i]);
 }
 
 __global__ void MergeNodesKernel(const DevNode *in, int64_t n, MergeOffsets off, DevNode *out) {
