@@ -1313,23 +1313,24 @@ int muon_gpu_intersect_arrays(MuonScene *scene, const float *origins, const floa
     scene->ray_out.Ensure(n * 8 * f);
     float *o = scene->ray_in.as<float>(), *d = o + 3 * n;
     float *dist = scene->ray_out.as<float>(), *id = dist + n, *pos = dist + 2 * n, *nrm = dist + 5 * n;
-    std::vector<float> stage(n <= kQueryStaged ? 8 * n : 0);
-    SendRays(scene, origins, directions, nullptr, n, stage.data());
+    std::vector<float> staged(n <= kQueryStaged ? 8 * n : 0);
+    float *stage = n <= kQueryStaged ? staged.data() : nullptr;
+    SendRays(scene, origins, directions, nullptr, n, stage);
     IntersectOnDevice(scene, QueryRays{o, d, 3}, n, intersect_mode,
                       QueryHits{dist, reinterpret_cast<int32_t *>(id), pos, nrm, 1, 3});
-    if (stage.empty()) {
+    if (!stage) {
       CUDA_TRY(cudaMemcpyAsync(distance, dist, n * f, cudaMemcpyDeviceToHost, st));
       CUDA_TRY(cudaMemcpyAsync(prim_id, id, n * f, cudaMemcpyDeviceToHost, st));
       CUDA_TRY(cudaMemcpyAsync(position, pos, 3 * n * f, cudaMemcpyDeviceToHost, st));
       CUDA_TRY(cudaMemcpyAsync(normal, nrm, 3 * n * f, cudaMemcpyDeviceToHost, st));
       CUDA_TRY(cudaStreamSynchronize(st));
     } else {
-      CUDA_TRY(cudaMemcpyAsync(stage.data(), dist, 8 * n * f, cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaMemcpyAsync(stage, dist, 8 * n * f, cudaMemcpyDeviceToHost, st));
       CUDA_TRY(cudaStreamSynchronize(st));
-      std::memcpy(distance, stage.data(), n * f);
-      std::memcpy(prim_id, stage.data() + n, n * f);
-      std::memcpy(position, stage.data() + 2 * n, 3 * n * f);
-      std::memcpy(normal, stage.data() + 5 * n, 3 * n * f);
+      std::memcpy(distance, stage, n * f);
+      std::memcpy(prim_id, stage + n, n * f);
+      std::memcpy(position, stage + 2 * n, 3 * n * f);
+      std::memcpy(normal, stage + 5 * n, 3 * n * f);
     }
   } catch (const CudaError &e) {
     return FailCuda(e);
@@ -1371,8 +1372,8 @@ int muon_gpu_occluded_arrays(MuonScene *scene, const float *origins, const float
     cudaStream_t st = scene->stream;
     scene->ray_in.Ensure(n * 7 * sizeof(float));
     scene->ray_out.Ensure(n);
-    std::vector<float> stage(n <= kQueryStaged ? 7 * n : 0);
-    SendRays(scene, origins, directions, max_distance, n, stage.data());
+    std::vector<float> staged(n <= kQueryStaged ? 7 * n : 0);
+    SendRays(scene, origins, directions, max_distance, n, n <= kQueryStaged ? staged.data() : nullptr);
     const float *o = scene->ray_in.as<float>();
     OccludedOnDevice(scene, QueryRays{o, o + 3 * n, 3}, o + 6 * n, n, intersect_mode, scene->ray_out.as<uint8_t>());
     CUDA_TRY(cudaMemcpyAsync(occluded, scene->ray_out.ptr, n, cudaMemcpyDeviceToHost, st));
