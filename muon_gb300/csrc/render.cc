@@ -645,11 +645,11 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   // traversal launch, the last blocks of a pass), the other's fill the SMs.
   // Films are still added in wave order. Per-kernel timing, probes and guiding
   // run the wavefronts one after another.
-  const bool in_pairs = MUON_WAVES_IN_FLIGHT > 1 && !timing && !probe && !guide && (bounded || pt);
+  const bool plain = !timing && !probe && !guide;
   const WavePlan plan = PlanWaves(W, H, p, budget);
   std::vector<WaveInfo> waves(plan.Count());
   for (size_t i = 0; i < waves.size(); ++i) waves[i] = plan.At(i);
-  const bool concurrent = in_pairs && waves.size() > 1;
+  const bool concurrent = MUON_WAVES_IN_FLIGHT > 1 && plain && waves.size() > 1;
   bool moved = sc->EnsureWork(std::min<int64_t>(plan.pix_per_wave, npix_total) * plan.ns, slots, concurrent ? 2 : 1);
   moved |= sc->EnsureCounters(stride * waves.size());
   sc->stats.Ensure(sizeof(unsigned long long) * kNumStats);
@@ -660,7 +660,7 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   // The next bounce's rays are traced beside a bounce's shadow rays and fold:
   // both follow from its shading, and where one's queue runs out the other
   // fills the chip (or, with short queues, hides its latency).
-  const bool lagged = !bounded && in_pairs;
+  const bool lagged = !bounded && plain;
   const bool overlap = pt && bounces > 1 && !timing && !probe && (bounded || lagged);
   if (overlap) sc->EnsureSide(last_set + 1);
   if (probe) {
@@ -790,8 +790,9 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
       // One or two wavefronts at a time, bounce by bounce. The host learns of a
       // queue's length while the next bounce already runs: a wavefront ends
       // with one bounce that finds no path.
-      for (size_t first = 0; first < waves.size(); first += 2) {
-        const size_t last = std::min(waves.size(), first + 2);
+      const size_t at_once = concurrent ? 2 : 1;
+      for (size_t first = 0; first < waves.size(); first += at_once) {
+        const size_t last = std::min(waves.size(), first + at_once);
         bool on[2] = {false, false};
         for (size_t wi = first; wi < last; ++wi) begin_wave(wi), on[wi & 1] = true;
         for (int k = 0; k < wave_bounces && (on[0] || on[1]); ++k) {
