@@ -35,7 +35,7 @@ def test_both_variants_find_the_same_hits(lib, deep, mode, depth):
     batch.close()
     assert np.array_equal(film.sum, full.sum) and np.array_equal(film.sum_sq, full.sum_sq)
     assert np.array_equal(film.count, full.count)
-    assert (film.sum > 0).any(axis=-1).mean() > 0.3
+    assert (film.sum > 0).any(axis=-1).mean() > 0.1  # (the slit room is dark)
 
 
 @pytest.mark.gpu
