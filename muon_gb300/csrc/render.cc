@@ -599,6 +599,21 @@ struct QueueProbe {
   }
 };
 
+// A guide's part of a frame graph's key: everything that the captured kernels
+// were given. A guide may lie where a destroyed one lay in part only, and a
+// graph of that one would write to its freed arrays.
+std::string GuideKey(const GuideDev &g) {
+  static_assert(sizeof(GuideDev) == 144, "every member is in the key");
+  char buf[512];
+  std::snprintf(buf, sizeof(buf),
+                " guide %p %p %p %p %p %p %p %p %p %p %zu %u %d %d %d %d %d %.9g %.9g %.9g %.9g %.9g %.9g %.9g", g.wt,
+                (void *)g.status, (void *)g.mix, (void *)g.feat, (void *)g.rec, (void *)g.pool, (void *)g.pool_count,
+                (void *)g.sample_count, (void *)g.sample_off, g.scan_tmp, g.scan_bytes, g.pool_cap, g.rec_cap,
+                g.rec_bounces, g.area_slots, g.mis_slot, g.direct_only, g.alpha, g.lo[0], g.lo[1], g.lo[2],
+                g.inv_ext[0], g.inv_ext[1], g.inv_ext[2]);
+  return buf;
+}
+
 // Renders into a device film. Throws CudaError.
 //
 // Bounded depth: every wavefront is a fixed launch sequence (camera; per
@@ -842,20 +857,18 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   cudaEvent_t t0 = sc->NextEvent(2)->a;
   cudaEvent_t t1 = sc->events[0].b;
   char keybuf[640];
-  int klen = std::snprintf(keybuf, sizeof(keybuf), "%d %d %d %d %d %d %d %d %d %d %llu %d %d %u %p %p %p %zu %d",
-                           p.integrator, p.pixel_samples, p.light_samples, p.light_stratify, p.next_event_estimation,
-                           p.russian_roulette, p.importance_sampling, p.min_depth, p.max_depth, p.sample_offset,
-                           (unsigned long long)p.seed, p.intersect_mode, p.wave_paths, p.flags, (void *)d_sum,
-                           (void *)d_sq, (void *)d_cnt, waves.size(), bounces);
-  if (guide && klen > 0 && klen < static_cast<int>(sizeof(keybuf)))
-    std::snprintf(keybuf + klen, sizeof(keybuf) - klen, " guide %p %p %p %p %d %d %.9g %.9g %.9g %.9g", guide->wt,
-                  (void *)guide->mix, (void *)guide->rec, (void *)guide->pool, guide->rec_cap, guide->rec_bounces,
-                  guide->alpha, guide->lo[0], guide->lo[1], guide->inv_ext[0]);
+  std::snprintf(keybuf, sizeof(keybuf), "%d %d %d %d %d %d %d %d %d %d %llu %d %d %u %p %p %p %zu %d", p.integrator,
+                p.pixel_samples, p.light_samples, p.light_stratify, p.next_event_estimation, p.russian_roulette,
+                p.importance_sampling, p.min_depth, p.max_depth, p.sample_offset, (unsigned long long)p.seed,
+                p.intersect_mode, p.wave_paths, p.flags, (void *)d_sum, (void *)d_sq, (void *)d_cnt, waves.size(),
+                bounces);
+  std::string key = keybuf;
+  if (guide) key += GuideKey(guide_local);
   const bool use_graph = bounded && !(p.flags & MUON_RENDER_NO_GRAPH) && !probe;
   if (moved) sc->DropGraph();
   CUDA_TRY(cudaEventRecord(t0, st));
-  const bool graph_ready = use_graph && sc->graph && sc->graph_key == keybuf;
-  if (graph_ready || (use_graph && sc->seen_key == keybuf)) {
+  const bool graph_ready = use_graph && sc->graph && sc->graph_key == key;
+  if (graph_ready || (use_graph && sc->seen_key == key)) {
     if (!graph_ready) {
       sc->DropGraph();
       cudaGraph_t g = nullptr;
@@ -875,7 +888,7 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
       cudaError_t e = cudaGraphInstantiate(&sc->graph, g, 0);
       cudaGraphDestroy(g);
       if (e != cudaSuccess) throw CudaError{e, "cudaGraphInstantiate"};
-      sc->graph_key = keybuf;
+      sc->graph_key = key;
       sc->graph_events = timed_pairs;
       sc->graph_launches = launches;
     }
@@ -884,7 +897,7 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
     timed_pairs = sc->graph_events;
   } else {
     enqueue(!bounded);
-    if (use_graph) sc->seen_key = keybuf;
+    if (use_graph) sc->seen_key = key;
   }
   CUDA_TRY(cudaEventRecord(t1, st));
   CUDA_TRY(cudaGetLastError());
