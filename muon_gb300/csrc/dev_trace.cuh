@@ -62,21 +62,13 @@ __device__ __forceinline__ float Min3(float a, float b, float c) {
 // Primitive records (64 bytes, 64-byte aligned) read with two 256-bit loads
 // instead of four 128-bit ones, as nodes are (TestChildren): half the load
 // requests to L1.
-#ifndef MUON_LD256
-#define MUON_LD256 1
-#endif
 __device__ __forceinline__ void Load64B(const void *p, float4 &a, float4 &b, float4 &c, float4 &d) {
-#if MUON_LD256
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
       : "l"(p));
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(c.x), "=f"(c.y), "=f"(c.z), "=f"(c.w), "=f"(d.x), "=f"(d.y), "=f"(d.z), "=f"(d.w)
       : "l"(static_cast<const char *>(p) + 32));
-#else
-  const float4 *q = static_cast<const float4 *>(p);
-  a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3);
-#endif
 }
 
 __device__ __forceinline__ float SafeInv(float x) {

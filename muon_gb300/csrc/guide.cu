@@ -450,38 +450,30 @@ __global__ void __launch_bounds__(kThreads, 2) WgradSquareKernel(const float *x,
   if (tid < 64) p[64 * 64 + tid] = sums[tid][64];
 }
 
-// The same for the first layer, whose inputs are the one-blob encoding.
-// Each thread owns a TK x TN tile of the K x N gradient; 32 samples at a time
-// are staged in shared memory (rows of K and N floats, read back as vectors).
-template <bool kBlob, int K, int N, int TK, int TN>
-__global__ void __launch_bounds__(kThreads) WgradKernel(const float *x, const float *dz, int batch, int chunk,
-                                                        float *partial, int stride, int layer_off) {
-  static_assert((K / TK) * (N / TN) == kThreads, "thread tiling");
-  static_assert(K % 4 == 0 && N % 4 == 0, "rows of whole 16-byte vectors");
+// The same for the first layer, whose inputs are the one-blob encoding: each
+// thread owns an 8 x 8 tile of the 256 x 64 gradient; 32 samples at a time are
+// staged in shared memory (rows of inputs and of outputs, read back as vectors).
+__global__ void __launch_bounds__(kThreads) WgradBlobKernel(const float *features, const float *dz, int batch,
+                                                            int chunk, float *partial, int layer_off) {
+  constexpr int K = kIn, N = kWidth, T = 8;
+  static_assert((K / T) * (N / T) == kThreads, "thread tiling");
   __shared__ __align__(16) float xs[32][K];
   __shared__ __align__(16) float ds[32][N];
-  __shared__ float fs[32][kFeatures];  // one-blob input: the slab's features
+  __shared__ float fs[32][kFeatures];  // the slab's features
   const int tid = threadIdx.x;
-  const int kg = tid / (N / TN), ng = tid % (N / TN);
+  const int kg = tid / (N / T), ng = tid % (N / T);
   const int b0 = blockIdx.x * chunk;
-  float acc[TK][TN] = {};
+  float acc[T][T] = {};
   float bacc = 0.0f;
   for (int s0 = b0; s0 < b0 + chunk && s0 < batch; s0 += 32) {
-    if (kBlob) {
-      for (int i = tid; i < 32 * kFeatures; i += kThreads) {
-        const int r = i / kFeatures, b = s0 + r;
-        fs[r][i % kFeatures] = b < batch ? x[static_cast<int64_t>(b) * kFeatures + i % kFeatures] : 0.0f;
-      }
-      __syncthreads();
+    for (int i = tid; i < 32 * kFeatures; i += kThreads) {
+      const int r = i / kFeatures, b = s0 + r;
+      fs[r][i % kFeatures] = b < batch ? features[static_cast<int64_t>(b) * kFeatures + i % kFeatures] : 0.0f;
     }
+    __syncthreads();
     for (int i = tid; i < 32 * K; i += kThreads) {
       const int r = i / K, k = i % K, b = s0 + r;
-      float v = 0.0f;
-      if (b < batch) {
-        if (kBlob) v = Blob(fs[r][k / kBins], k % kBins);
-        else v = x[static_cast<int64_t>(b) * K + k];
-      }
-      xs[r][k] = v;
+      xs[r][k] = b < batch ? Blob(fs[r][k / kBins], k % kBins) : 0.0f;
     }
     for (int i = tid; i < 32 * N; i += kThreads) {
       const int r = i / N, n = i % N, b = s0 + r;
@@ -490,23 +482,23 @@ __global__ void __launch_bounds__(kThreads) WgradKernel(const float *x, const fl
     __syncthreads();
 #pragma unroll 4
     for (int r = 0; r < 32; ++r) {
-      float a[TK], d[TN];
-      LoadRow<TK>(&xs[r][kg * TK], a);
-      LoadRow<TN>(&ds[r][ng * TN], d);
+      float a[T], d[T];
+      LoadRow<T>(&xs[r][kg * T], a);
+      LoadRow<T>(&ds[r][ng * T], d);
 #pragma unroll
-      for (int i = 0; i < TK; ++i)
+      for (int i = 0; i < T; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] += a[i] * d[j];
+        for (int j = 0; j < T; ++j) acc[i][j] += a[i] * d[j];
     }
     if (tid < N)
       for (int r = 0; r < 32; ++r) bacc += ds[r][tid];
     __syncthreads();
   }
-  float *p = partial + static_cast<int64_t>(blockIdx.x) * stride + layer_off;
+  float *p = partial + static_cast<int64_t>(blockIdx.x) * kParams + layer_off;
 #pragma unroll
-  for (int i = 0; i < TK; ++i)
+  for (int i = 0; i < T; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) p[(kg * TK + i) * N + ng * TN + j] = acc[i][j];
+    for (int j = 0; j < T; ++j) p[(kg * T + i) * N + ng * T + j] = acc[i][j];
   if (tid < N) p[K * N + tid] = bacc;
 }
 
@@ -656,8 +648,7 @@ void LaunchGuideGradients(const float *params, const float *features, const floa
     cur ^= 1;
   }
   // layer 0: one-blob input, 256 x 64
-  WgradKernel<true, kIn, kWidth, 8, 8><<<chunks, kThreads, 0, st>>>(features, dz, batch, chunk, tb.partial, kParams,
-                                                                    MasterOffset(0));
+  WgradBlobKernel<<<chunks, kThreads, 0, st>>>(features, dz, batch, chunk, tb.partial, MasterOffset(0));
   ReduceKernel<<<Grid(kParams, 256), 256, 0, st>>>(tb.partial, tb.chunks, tb.grad);
 }
 
