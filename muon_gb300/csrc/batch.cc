@@ -117,10 +117,12 @@ struct MuonBatch {
     return b;
   }
 
-  bool EnsureWork(int64_t paths, int slots) {
-    if (paths <= wave_cap && slots <= slots_cap) return false;
+  void EnsureWork(int64_t paths, int slots) {
+    if (paths <= wave_cap && slots <= slots_cap) return;
     int64_t p = std::max(paths, wave_cap);
     int s = std::max(slots, slots_cap);
+    DropGraph();                   // it holds the old addresses
+    wave_cap = 0, slots_cap = -1;  // nothing to use until every array has grown
     for (int k = 0; k < 2; ++k) {
       ray_o[k].Ensure(p * sizeof(float4));
       ray_d[k].Ensure(p * sizeof(float4));
@@ -138,7 +140,6 @@ struct MuonBatch {
     order.Ensure(static_cast<size_t>(OrderInts(p)) * sizeof(int32_t));
     wave_cap = p;
     slots_cap = s;
-    return true;
   }
 };
 
@@ -336,11 +337,11 @@ void RenderBatch(MuonBatch *b, const MuonRenderParams *params, double *const *d_
     s.sum_sq = d_sq[i];
     s.count = d_cnt[i];
   }
-  bool moved = b->EnsureWork(budget, S);
+  b->EnsureWork(budget, S);
   const size_t table_bytes = scenes.size() * sizeof(BatchScene), seg_bytes = segs.size() * sizeof(BatchSeg);
   if (b->scene_table.bytes < table_bytes || b->seg_table.bytes < seg_bytes ||
       b->counters.bytes < stride * waves.size() * sizeof(uint32_t))
-    moved = true;
+    b->DropGraph();
   b->scene_table.Ensure(table_bytes);
   b->seg_table.Ensure(seg_bytes);
   b->counters.Ensure(stride * waves.size() * sizeof(uint32_t));
@@ -426,7 +427,6 @@ void RenderBatch(MuonBatch *b, const MuonRenderParams *params, double *const *d_
       key += buf;
     }
   }
-  if (moved) b->DropGraph();
   if (b->graph_key != key || !b->graph) {
     b->DropGraph();
     SetTraversalBlocksOverride(b->blocks_per_sm > 0 ? b->blocks_per_sm * b->sms : 0);

@@ -48,11 +48,13 @@ struct WorkSet {
   int64_t cap = 0;
   int slots = -1;
 
-  // Grows the arrays (the scene's streams are idle); true if any moved.
-  bool Ensure(int64_t paths, int slots_wanted, int device) {
-    if (paths <= cap && slots_wanted <= slots) return false;
+  bool Has(int64_t paths, int slots_wanted) const { return paths <= cap && slots_wanted <= slots; }
+
+  // Grows the arrays (the scene's streams are idle).
+  void Ensure(int64_t paths, int slots_wanted, int device) {
     const int64_t p = std::max(paths, cap);
     const int sl_count = std::max(slots_wanted, slots);
+    cap = 0, slots = -1;  // nothing to use until every array has grown
     for (int k = 0; k < 2; ++k) {
       EnsurePooled(ray_o[k], p * sizeof(float4), device);
       EnsurePooled(ray_d[k], p * sizeof(float4), device);
@@ -70,7 +72,6 @@ struct WorkSet {
     EnsurePooled(order, static_cast<size_t>(OrderInts(p)) * sizeof(int32_t), device);
     cap = p;
     slots = sl_count;
-    return true;
   }
 
   // The arrays as bounce `bounce` uses them: hits and links alternate, so that
@@ -193,11 +194,14 @@ struct MuonScene {
 
   PathBuffers Buffers(int set, int bounce) const { return work[set].Buffers(stats, bounce); }
 
-  // Grows the path arrays of `sets` wavefronts in flight; true if any moved.
-  bool EnsureWork(int64_t paths, int slots, int sets = 1) {
-    bool moved = false;
-    for (int k = 0; k < sets; ++k) moved |= work[k].Ensure(paths, slots, device);
-    return moved;
+  // Grows the path arrays of `sets` wavefronts in flight; a graph that holds
+  // their old addresses goes, also where an allocation fails.
+  void EnsureWork(int64_t paths, int slots, int sets = 1) {
+    for (int k = 0; k < sets; ++k)
+      if (!work[k].Has(paths, slots)) {
+        DropGraph();
+        work[k].Ensure(paths, slots, device);
+      }
   }
 
   // The second stream and the events that order two wavefronts in flight.
@@ -219,16 +223,16 @@ struct MuonScene {
     }
   }
 
-  // Grows the device and pinned host counter arrays; returns true if the
-  // device pointer changed.
-  bool EnsureCounters(size_t words) {
-    if (words <= h_counters_len) return false;
+  // Grows the device and pinned host counter arrays (as EnsureWork).
+  void EnsureCounters(size_t words) {
+    if (words <= h_counters_len) return;
+    DropGraph();
+    h_counters_len = 0;
     counters.Ensure(words * sizeof(uint32_t));
     if (h_counters) cudaFreeHost(h_counters);
     h_counters = nullptr;
     CUDA_TRY(cudaMallocHost(reinterpret_cast<void **>(&h_counters), words * sizeof(uint32_t)));
     h_counters_len = words;
-    return true;
   }
 
   void DropGraph() {
@@ -253,6 +257,7 @@ int Fail(int code, const std::string &msg) {
   return code;
 }
 int FailCuda(const CudaError &e) {
+  cudaGetLastError();  // the next call checks its own launches
   return Fail(MUON_ERR_CUDA, std::string(e.where) + ": " + cudaGetErrorString(e.code));
 }
 
@@ -665,8 +670,8 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   std::vector<WaveInfo> waves(plan.Count());
   for (size_t i = 0; i < waves.size(); ++i) waves[i] = plan.At(i);
   const bool concurrent = MUON_WAVES_IN_FLIGHT > 1 && plain && waves.size() > 1;
-  bool moved = sc->EnsureWork(std::min<int64_t>(plan.pix_per_wave, npix_total) * plan.ns, slots, concurrent ? 2 : 1);
-  moved |= sc->EnsureCounters(stride * waves.size());
+  sc->EnsureWork(std::min<int64_t>(plan.pix_per_wave, npix_total) * plan.ns, slots, concurrent ? 2 : 1);
+  sc->EnsureCounters(stride * waves.size());
   sc->stats.Ensure(sizeof(unsigned long long) * kNumStats);
   if (concurrent || !bounded) sc->EnsureStream2();
   const int last_set = concurrent ? 1 : 0;
@@ -865,7 +870,6 @@ void RenderDevice(MuonScene *sc, const MuonRenderParams &p, double *d_sum, doubl
   std::string key = keybuf;
   if (guide) key += GuideKey(guide_local);
   const bool use_graph = bounded && !(p.flags & MUON_RENDER_NO_GRAPH) && !probe;
-  if (moved) sc->DropGraph();
   CUDA_TRY(cudaEventRecord(t0, st));
   const bool graph_ready = use_graph && sc->graph && sc->graph_key == key;
   if (graph_ready || (use_graph && sc->seen_key == key)) {
