@@ -625,8 +625,9 @@ std::string GuideKey(const GuideDev &g) {
 // bounce extend, shade, occlude, fold; film) whose kernels read their queue
 // lengths from device counters, so the whole frame is captured once into a
 // CUDA graph and replayed; the host synchronises once per frame. Unbounded
-// depth (max_depth -1): the host reads the queue length after every bounce and
-// stops when no path continues.
+// depth (max_depth -1): the host reads a bounce's queue length while the next one
+// runs and stops when no path continues (with per-kernel timing, probes and
+// guiding, after every bounce).
 // Wavefronts in flight at a time in a render (1 or 2).
 #ifndef MUON_WAVES_IN_FLIGHT
 #define MUON_WAVES_IN_FLIGHT 2
